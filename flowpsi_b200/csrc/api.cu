@@ -427,6 +427,12 @@ int fpsi_create(fpsi_ctx** out, const fpsi_mesh* mesh, const fpsi_params* params
     delete x;
     return FPSI_E_CUDA;
   }
+  if (cudaGetDevice(&x->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&x->nsm, cudaDevAttrMultiProcessorCount, x->device) != cudaSuccess) {
+    fpsi::set_error("device query failed");
+    fpsi_destroy(x);
+    return FPSI_E_CUDA;
+  }
   TRY(upload(x, &x->d_cl, H.cl));
   TRY(upload(x, &x->d_cr, H.cr));
   TRY(upload(x, &x->d_n, soa3(H.n, nf)));

@@ -126,6 +126,7 @@ struct fpsi_ctx {
   fpsi::HostMesh H;
   std::vector<fpsi_bc> bcs;
   int device = 0;
+  int nsm = 148;  // multiprocessors of the device
   cudaStream_t stream = nullptr;
   // ---- device arrays (new numbering) ----
   // geometry

@@ -1692,6 +1692,19 @@ __global__ void k_jacobi_start(ColInfo ck, const TB* __restrict__ luc,
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch: a grid launched with launch_after may start
+// while the grid before it drains; what it touches before pdl_wait must not
+// be written by any grid that can still be running.  Both are no-ops in a
+// plain launch.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+constexpr int SGS_THREADS = 128;
+
+// ---------------------------------------------------------------------------
 // one colour of a Gauss-Seidel sweep (gseidel_forward/backward,
 // linearSolverSGS.loci:186-207, 277-298):
 //   x_c = D^-1 (B - sum_upper fjm x_cr + sum_lower fjp x_cl)
@@ -1703,17 +1716,69 @@ __global__ void k_jacobi_start(ColInfo ck, const TB* __restrict__ luc,
 // iterate, which every colour re-reads, stays resident in L2.
 // CPT: slots hold the compact form (CK_SLOT values), applied without
 // spelling out the 25 entries.
+//
+// The passes of a solve form one serial chain of short grids, so each pass
+// is launched while the one before it drains (programmatic dependent
+// launch): everything the sweep does not write -- LU, pivots, B, neighbour
+// ids and the first slots' blocks -- is requested before the wait for the
+// previous pass, and only the iterate after it.  Large passes are bound by HBM (400 B per cell of the compact
+// FP32 form: 24 us a pass of 393 k cells at the copy rate), small ones by
+// the launch and the dependent loads.  A step of 8 sweeps over 24,576 tets
+// went from 0.283 to 0.163 ms, 196,608 from 0.562 to 0.390, 663,552 from 1.20
+// to 1.04, 1.57 M from 2.61 to 2.48, 12.6 M from 19.9 to 19.7 (MIXED); 32,768
+// viscous hexes with explicit blocks from 0.482 to 0.200.
+//
+// MS: slots walked with their neighbour iterates and the first sgs_ahead()
+// blocks in flight together (4 covers tets, 6 hexes and prisms), at the
+// registers that takes; 0: any number of slots one after the other, few
+// registers and more CTAs per SM.  launch_sgs_pass picks MS > 0 where the
+// grid fits on the device in one wave (24,576 tets REF: 0.217 ms a step
+// against 0.296 slot by slot) and for FP32 tets of any size (663,552 cells:
+// 1.050 against 1.053, 1.57 M 2.481 against 2.525); larger grids of the
+// other forms stream faster slot by slot (592,704 hexes MIXED 1.00 against
+// 1.09, 663,552 tets FP64 1.65 against 1.90).
+template <class TB, class TX, bool CPT, int MS>
+constexpr int sgs_ahead() {
+  return MS == 0 ? 0 : sizeof(TB) == 4 ? (CPT ? 4 : 2) : (CPT ? 1 : 0);
+}
+template <class TB, class TX, bool CPT, int MS>
+constexpr int sgs_ctas() {  // CTAs per SM the registers are limited for
+  if (MS == 0) return sizeof(TX) == 4 ? 8 : sizeof(TB) == 4 ? (CPT ? 6 : 5) : 4;
+  return sizeof(TX) == 4 ? (CPT && MS == 6 ? 3 : 4) : sizeof(TB) == 4 ? 3 : 2;
+}
+__device__ __forceinline__ void hold(float& v) { asm volatile("" : "+f"(v)); }
 template <class TB, class TX, bool CPT>
-__global__ void k_sgs_colour(ColInfo ck, const int32_t* __restrict__ nbr,
-                             const TB* __restrict__ aoff, const TB* __restrict__ luc,
-                             const TB* __restrict__ bcv, const int32_t* __restrict__ pvv,
-                             TX* __restrict__ x) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void sgs_slot(const TB* A, const TX* xv, TX* t) {
+  if constexpr (CPT) {
+    compact_apply<TB, TX>(A, xv, t);
+  } else {
+#pragma unroll
+    for (int r = 0; r < 5; ++r)
+#pragma unroll
+      for (int j = 0; j < 5; ++j) t[r] += TX(A[5 * r + j]) * xv[j];
+  }
+}
+template <class TB, class TX, bool CPT, int MS>
+__global__ void __launch_bounds__(SGS_THREADS, sgs_ctas<TB, TX, CPT, MS>())
+k_sgs_colour(ColInfo ck, const int32_t* __restrict__ nbr, const TB* __restrict__ aoff,
+             const TB* __restrict__ luc, const TB* __restrict__ bcv, const int32_t* __restrict__ pvv,
+             TX* x) {
+  constexpr int SW = CPT ? CK_SLOT : 25;  // values per slot
+  constexpr int AH = sgs_ahead<TB, TX, CPT, MS>();
+  pdl_trigger();
+  const int64_t i = int64_t(blockIdx.x) * SGS_THREADS + threadIdx.x;
   const int64_t n = ck.n, ld = ck.ld;
   if (i >= n) return;
-  // the cell's LU factors and pivots are loaded first, so that they are in
-  // flight while the slots are walked; each slot's neighbour id is read one
-  // slot ahead
+  const int m = int(ck.m);
+  const int32_t* nb = nbr + ck.ebp + i;
+  const TB* A = aoff + SW * ck.ebp + i;
+  int32_t o[MS > 0 ? MS : 1];
+  if constexpr (MS > 0) {
+#pragma unroll
+    for (int s = 0; s < MS; ++s) o[s] = s < m ? __ldcs(nb + s * ld) : -1;
+  } else {
+    o[0] = m > 0 ? __ldcs(nb) : -1;
+  }
   TB LU[25];
 #pragma unroll
   for (int k = 0; k < 25; ++k) LU[k] = __ldcs(luc + 25 * ck.cbp + k * ld + i);
@@ -1721,26 +1786,57 @@ __global__ void k_sgs_colour(ColInfo ck, const int32_t* __restrict__ nbr,
   TX t[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) t[k] = -TX(__ldcs(bcv + 5 * ck.cbp + k * ld + i));
-  int32_t o = ck.m > 0 ? __ldcs(nbr + ck.ebp + i) : -1;
-  for (int64_t s = 0; s < ck.m && o >= 0; ++s) {
-    const int32_t onext = s + 1 < ck.m ? __ldcs(nbr + ck.ebp + (s + 1) * ld + i) : -1;
-    TX xv[5];
+  TB ca[AH > 0 ? AH : 1][SW];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) xv[k] = x[5 * int64_t(o) + k];
-    if constexpr (CPT) {
-      const TB* A = aoff + CK_SLOT * ck.ebp + s * CK_SLOT * ld + i;
-      TB c[CK_SLOT];
+  for (int s = 0; s < AH; ++s)
+    if (s < m) {
 #pragma unroll
-      for (int k = 0; k < CK_SLOT; ++k) c[k] = __ldcs(A + k * ld);
-      compact_apply<TB, TX>(c, xv, t);
-    } else {
-      const TB* A = aoff + 25 * ck.ebp + s * 25 * ld + i;
-#pragma unroll
-      for (int r = 0; r < 5; ++r)
-#pragma unroll
-        for (int j = 0; j < 5; ++j) t[r] += TX(__ldcs(A + (5 * r + j) * ld)) * xv[j];
+      for (int k = 0; k < SW; ++k) ca[s][k] = __ldcs(A + (s * SW + k) * ld);
     }
-    o = onext;
+  pdl_wait();
+  // FP32 blocks under an FP64 iterate are widened where they are used, not
+  // while they wait (twice the registers)
+  if constexpr (sizeof(TB) < sizeof(TX)) {
+#pragma unroll
+    for (int k = 0; k < 25; ++k) hold(LU[k]);
+#pragma unroll
+    for (int s = 0; s < AH; ++s)
+#pragma unroll
+      for (int k = 0; k < SW; ++k) hold(ca[s][k]);
+  }
+  if constexpr (MS > 0) {
+    TX xv[MS][5];
+#pragma unroll
+    for (int s = 0; s < MS; ++s)
+      if (o[s] >= 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) xv[s][k] = x[5 * int64_t(o[s]) + k];
+      }
+#pragma unroll
+    for (int s = 0; s < MS; ++s) {
+      if (o[s] < 0) continue;  // a cell's slots are filled from the first
+      if (s < AH) {
+        sgs_slot<TB, TX, CPT>(ca[s < AH ? s : 0], xv[s], t);
+      } else {
+        TB c[SW];
+#pragma unroll
+        for (int k = 0; k < SW; ++k) c[k] = __ldcs(A + (s * SW + k) * ld);
+        sgs_slot<TB, TX, CPT>(c, xv[s], t);
+      }
+    }
+  } else {
+    int32_t os = o[0];
+    for (int s = 0; s < m && os >= 0; ++s) {
+      const int32_t onext = s + 1 < m ? __ldcs(nb + (s + 1) * ld) : -1;
+      TX xv[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) xv[k] = x[5 * int64_t(os) + k];
+      TB c[SW];
+#pragma unroll
+      for (int k = 0; k < SW; ++k) c[k] = __ldcs(A + (int64_t(s) * SW + k) * ld);
+      sgs_slot<TB, TX, CPT>(c, xv, t);
+      os = onext;
+    }
   }
   TX y[5];
 #pragma unroll
@@ -2243,6 +2339,29 @@ int launch_jacobi_start(fpsi_ctx* x) {
   }
 }
 
+// one sweep pass; after: the grid before it on the stream is a sweep pass
+// too (a first pass waits for the assembly it reads in full)
+template <class TB, class TX, bool CPT, int MS>
+static cudaError_t launch_sgs_pass(fpsi_ctx* x, const ColInfo& ck, bool after) {
+  const int64_t grid = blocks_for(ck.n, dev::SGS_THREADS);
+  if constexpr (MS > 0 && !(sizeof(TX) == 4 && CPT && MS == 4)) {
+    if (grid > int64_t(dev::sgs_ctas<TB, TX, CPT, MS>()) * x->nsm)
+      return launch_sgs_pass<TB, TX, CPT, 0>(x, ck, after);
+  }
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(dev::SGS_THREADS);
+  cfg.stream = x->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, dev::k_sgs_colour<TB, TX, CPT, MS>, ck, (const int32_t*)x->d_nbr,
+                            (const TB*)x->d_aoff, (const TB*)x->d_luc, (const TB*)x->d_bc,
+                            (const int32_t*)x->d_pv, (TX*)x->d_x);
+}
+
 template <class TB, class TX>
 // Forward then backward over the colours, `sweeps` times.  A colour's cells
 // read only other colours' iterates, so a colour that directly follows
@@ -2250,8 +2369,6 @@ template <class TB, class TX>
 // would reproduce the values it just wrote: those launches are skipped and
 // the iterate is bitwise the same as with every launch made.
 static int launch_sgs_t(fpsi_ctx* x, int sweeps) {
-  cudaStream_t s = x->stream;
-  const int T = 128;
   const int K = x->H.ncolours;
   int last = -1;
   for (int it = 0; it < sweeps; ++it) {
@@ -2260,16 +2377,19 @@ static int launch_sgs_t(fpsi_ctx* x, int sweeps) {
         const int k = pass == 0 ? kk : K - 1 - kk;
         const ColInfo ck = col_info(x, k);
         if (ck.n == 0 || k == last) continue;
+        const bool after = last >= 0 && !x->profiling;
         last = k;
         prof_begin(x, "sgs_colour");
+        cudaError_t e;
         if (x->asm_compact)
-          dev::k_sgs_colour<TB, TX, true><<<blocks_for(ck.n, T), T, 0, s>>>(
-              ck, x->d_nbr, (const TB*)x->d_aoff, (const TB*)x->d_luc, (const TB*)x->d_bc, x->d_pv,
-              (TX*)x->d_x);
+          e = ck.m <= 4   ? launch_sgs_pass<TB, TX, true, 4>(x, ck, after)
+              : ck.m <= 6 ? launch_sgs_pass<TB, TX, true, 6>(x, ck, after)
+                          : launch_sgs_pass<TB, TX, true, 0>(x, ck, after);
         else
-          dev::k_sgs_colour<TB, TX, false><<<blocks_for(ck.n, T), T, 0, s>>>(
-              ck, x->d_nbr, (const TB*)x->d_aoff, (const TB*)x->d_luc, (const TB*)x->d_bc, x->d_pv,
-              (TX*)x->d_x);
+          e = ck.m <= 4   ? launch_sgs_pass<TB, TX, false, 4>(x, ck, after)
+              : ck.m <= 6 ? launch_sgs_pass<TB, TX, false, 6>(x, ck, after)
+                          : launch_sgs_pass<TB, TX, false, 0>(x, ck, after);
+        FPSI_CUDA_TRY(e);
         prof_end(x);
       }
   }

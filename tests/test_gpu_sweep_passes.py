@@ -1,0 +1,86 @@
+"""Sweep passes at the sizes where their variants change: less than one tile,
+whole tiles and a remainder, passes that fit the device in one wave and
+passes that do not, 4, 6 and more than 6 neighbours, compact and explicit
+blocks.  GPU only.  Against the oracle's sweeps in the same colour order,
+FP64: 1e-8 of the largest entry of each component (the diagonal blocks'
+condition numbers reach 1e6, FP64 rounding 1e-16, and the truncated sweeps
+amplify by less than 100); FP32 blocks: within twice the oracle's own FP32
+distance from its FP64 result plus 1e-6 of the largest entry."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from flowpsi_b200 import FlowPsi, _native as N, cases
+from oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+class PairedHexes:
+    """a hex farfield box whose cells 2c and 2c+1 are merged: up to ten faces
+    per cell"""
+
+    def __init__(self, case):
+        self.base, a = case.mesh, case.mesh.arrays()  # owns the nodes and conditions
+        cl, cr = a.cl // 2, np.where(a.cr >= 0, a.cr // 2, a.cr)
+        keep = np.flatnonzero(cl != cr)
+        k = np.diff(a.face_off)
+        self.nodes = np.concatenate([a.face_nodes[a.face_off[f]:a.face_off[f + 1]] for f in keep])
+        self.off = np.concatenate([[0], np.cumsum(k[keep])]).astype(np.int64)
+        self.cl, self.cr = cl[keep].astype(np.int32), cr[keep].astype(np.int32)
+        m = N.Mesh()
+        m.nnodes, m.ncells, m.nfaces = self.base.m.nnodes, a.ncells // 2, len(keep)
+        m.xyz, m.nbc, m.bcs = self.base.m.xyz, self.base.m.nbc, self.base.m.bcs
+        m.face_off = self.off.ctypes.data_as(C.POINTER(C.c_int64))
+        m.face_nodes, m.cl, m.cr = N.iptr(self.nodes), N.iptr(self.cl), N.iptr(self.cr)
+        self.mesh = m
+
+
+def merged(n, prec):
+    c = cases.farfield_cube(n, precision=prec)
+    c.pairs = PairedHexes(c)  # keeps the arrays alive
+    c.mesh = c.pairs.mesh
+    return c
+
+
+CASES = {
+    "hex_4": lambda p: cases.farfield_cube(4, precision=p),      # 32 cells a pass
+    "hex_8": lambda p: cases.farfield_cube(8, precision=p),      # two whole tiles
+    "hex_49": lambda p: cases.farfield_cube(49, precision=p),    # more than one wave
+    "tets_7": lambda p: cases.farfield_tets(7, precision=p),     # remainders
+    "paired_6": lambda p: merged(6, p),                          # up to ten neighbours
+    "viscous_hex": lambda p: cases.boundary_layer_block(11, 9, 5, viscous=1, solver="sgs",
+                                                        precision=p, dy0=1e-3),
+}
+
+
+def _dq(maker, prec):
+    case = CASES[maker](prec)
+    o = Oracle(case.mesh, case.params)
+    st = case.initial_state(o.geometry()["cellcenter"])
+    o.set_state(*st)
+    o.residual()
+    o.assemble()
+    return case, st, o
+
+
+@pytest.mark.parametrize("prec", ["fp64", "ref", "mixed"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_sweeps_match_oracle(need_gpu, name, prec):
+    case, st, o = _dq(name, prec)
+    g = FlowPsi(case.mesh, case.params)
+    g.set_state(*st)
+    g.residual()
+    g.assemble()
+    col = g.colours()
+    dg, do = g.linear_solve(), o.linear_solve(colour=col)
+    if prec != "fp64":
+        d64 = _dq(name, "fp64")[2].linear_solve(colour=col)
+    for k in range(5):
+        if prec == "fp64":
+            assert np.abs(dg[:, k] - do[:, k]).max() <= 1e-8 * np.abs(do[:, k]).max(), k
+        else:
+            e_orc, e_gpu = (np.abs(d[:, k] - d64[:, k]).max() for d in (do, dg))
+            assert e_gpu <= 2.0 * e_orc + 1e-6 * np.abs(d64[:, k]).max(), k
+    g.close()
