@@ -103,7 +103,8 @@ struct fpsi_gnn {
   __nv_bfloat16 *d_h[NLAYER + 1] = {nullptr}, *d_agg[NLAYER] = {nullptr};
   float* d_z[NLAYER] = {nullptr};
   float *d_y = nullptr, *d_dh = nullptr, *d_dh2 = nullptr, *d_dz = nullptr, *d_dagg = nullptr;
-  float* d_part = nullptr;  // weight-gradient partials
+  float* d_part = nullptr;  // weight-gradient partials of part_cap CTAs
+  int64_t part_cap = 0;
   double* d_lpart = nullptr;
   std::vector<Snapshot> snaps;
   cudaStream_t stream = nullptr;
@@ -141,9 +142,6 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return sg + x * sg * (1.0f - sg) * (2.0f * GELU_K) * fmaf(3.0f * GELU_C, x2, 1.0f);
 }
 
-// a layer input as the tensor cores multiply it (FP32 features rounded to BF16)
-__device__ __forceinline__ float as_operand(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__device__ __forceinline__ float as_operand(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 // ---- tcgen05 helpers (single-CTA MMA, no multicast) ----------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -845,13 +843,6 @@ __global__ void __launch_bounds__(GT) k_loss(int64_t nc, const float* __restrict
   if (threadIdx.x == 0) part[2 * blockIdx.x] = s1[0], part[2 * blockIdx.x + 1] = s2[0];
 }
 
-__global__ void k_scale(int64_t n, float* __restrict__ a, const double* __restrict__ loss_cnt) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double cnt = loss_cnt[1];
-  a[i] = float(double(a[i]) * (cnt > 0 ? 2.0 / (5.0 * cnt) : 0.0));
-}
-
 // sum of the loss partials: out[0] = mean squared error, out[1] = batch size
 __global__ void k_loss_final(const double* __restrict__ part, int nblk, double* __restrict__ out) {
   __shared__ double s1[256], s2[256];
@@ -869,89 +860,290 @@ __global__ void k_loss_final(const double* __restrict__ part, int nblk, double* 
   }
 }
 
-// weight-gradient partials over blocks of RB cells:
-// part[blk][j][i] = sum_c dz[c][j] * a[c][i]   (a = h or agg, as the forward
-// GEMM used it), and bias sums
-constexpr int RB = 256;
-template <class TA>
-__global__ void k_wgrad_partial(int64_t nc, int nout, int fin, const float* __restrict__ dz,
-                                const TA* __restrict__ a, float* __restrict__ part) {
-  const int64_t c0 = int64_t(blockIdx.x) * RB;
-  const int64_t c1 = min(nc, c0 + RB);
-  float* o = part + int64_t(blockIdx.x) * nout * (fin + 1);
-  for (int w = threadIdx.x; w < nout * (fin + 1); w += blockDim.x) {
-    const int j = w / (fin + 1), i = w % (fin + 1);
-    float s = 0.f;
-    if (i < fin) {
-      for (int64_t c = c0; c < c1; ++c) s += dz[c * nout + j] * as_operand(a[c * fin + i]);
+// One layer of the backward pass, a CTA per rb cells (whole tiles of BT):
+//   dh  = Wo^T dy (TOP: the last layer, under the head), else the layer
+//         above's dh_in + its neighbour part: sum_{c in N} dagg_in[c] / deg(c)
+//         (the graph is symmetric)
+//   dz  = dh GELU'(z)
+//   part: the CTA's sums over its cells of dz x [h | agg] and dz (and, TOP,
+//         of dy x h_out and dy)
+//   dh_out = dz Ws, dagg_out = dz Wn   (DENSE: every layer but the first)
+// The two products are FP32 FMAs: 16,384 per cell and hidden layer, which the
+// weights, dz and the layer's inputs feed from shared memory as 4 x 8 register
+// tiles, three 16 B loads per 32 FMAs.  Bound by the FMA pipe (ideal 0.2 ms
+// for 196,608 cells).  The layer's dz and its neighbour sums never reach
+// memory.  A loss-and-gradient call over 196,608 cells went from 5.68 to 1.14
+// ms (one thread per weight walking 256 cells before), over 1.57 M from 42.7
+// to 7.4; the neighbour gather of dagg_in is what keeps it from the FMA
+// rate.  Weight-gradient sums run over at most RB cells in FP32 in cell order
+// and across CTAs in FP64.
+constexpr int RB = 256;   // most cells per CTA and partial
+constexpr int BT = 64;    // cells per tile
+constexpr int BTH = 256;  // threads per CTA
+constexpr int BZS = 68;   // floats per staged dz row: 16 B aligned, rows on different banks
+// floats of one CTA's partial: [64][2 fin] (Ws | Wn), b, then Wo, bo
+constexpr int back_part(int fin, bool top) { return W * 2 * fin + W + (top ? NOUT * W + NOUT : 0); }
+struct BackSmem {  // floats
+  int dz, a, w, dy, red, total;
+};
+__host__ __device__ constexpr BackSmem back_smem(int fin, bool dense) {
+  BackSmem s{};
+  s.dz = 0;
+  s.a = s.dz + BT * BZS;
+  s.w = s.a + BT * 2 * fin;
+  s.dy = s.w + (dense ? W * 2 * fin : 0);
+  s.red = s.dy + BT * 8;
+  s.total = s.red + 4 * (W + NOUT * W + 8);
+  return s;
+}
+__device__ __forceinline__ void fma4(float4& a, float s, const float4& v) {
+  a.x = fmaf(s, v.x, a.x), a.y = fmaf(s, v.y, a.y), a.z = fmaf(s, v.z, a.z), a.w = fmaf(s, v.w, a.w);
+}
+template <int FIN, bool TOP, bool DENSE, class TA>
+__global__ void __launch_bounds__(BTH, 2)
+k_back_layer(int64_t nc, int rb, const int32_t* __restrict__ off, const int32_t* __restrict__ nb,
+             const float* __restrict__ z, const TA* __restrict__ h, const __nv_bfloat16* __restrict__ agg,
+             const __nv_bfloat16* __restrict__ ws, const __nv_bfloat16* __restrict__ wn,
+             const float* __restrict__ dh_in, const float* __restrict__ dagg_in,
+             const float* __restrict__ dy, const double* __restrict__ loss_cnt,
+             const __nv_bfloat16* __restrict__ wo, const __nv_bfloat16* __restrict__ hout,
+             float* __restrict__ dh_out, float* __restrict__ dagg_out, float* __restrict__ part) {
+  constexpr int NC = 2 * FIN;       // input columns: own | neighbour mean
+  constexpr int NI = NC / 16;       // columns per thread of the weight gradient
+  static_assert(NC % 16 == 0 && (!DENSE || FIN == W), "tile shapes");
+  extern __shared__ __align__(16) float bsm[];
+  constexpr BackSmem S = back_smem(FIN, DENSE);
+  float *sdz = bsm + S.dz, *sa = bsm + S.a, *sw = bsm + S.w, *sdy = bsm + S.dy, *sred = bsm + S.red;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (DENSE)
+    for (int i = t; i < W * NC; i += BTH) {
+      const int j = i / NC, k = i - NC * j;
+      sw[i] = __bfloat162float(k < FIN ? ws[j * FIN + k] : wn[j * FIN + k - FIN]);
+    }
+  const int jg = t >> 4, ig = t & 15;  // weight gradient: rows 4 jg.., columns of ig
+  float g[4][NI];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int k = 0; k < NI; ++k) g[r][k] = 0.f;
+  const int bj = t & 63, bq = t >> 6;  // bias and head sums: feature bj, quarter of the tile's cells
+  float gb = 0.f, gbo = 0.f, go[NOUT];
+#pragma unroll
+  for (int k = 0; k < NOUT; ++k) go[k] = 0.f;
+  double scale = 0.0;  // of dy, from the batch's size
+  if (TOP) scale = loss_cnt[1] > 0 ? 2.0 / (5.0 * loss_cnt[1]) : 0.0;
+  const int64_t c0 = int64_t(blockIdx.x) * rb;
+  for (int64_t t0 = c0; t0 < min(c0 + rb, nc); t0 += BT) {
+    __syncthreads();  // the tile before is done with the staging
+    if (TOP) {
+      for (int i = t; i < BT * NOUT; i += BTH) {
+        const int c = i / NOUT, k = i - NOUT * c;
+        sdy[8 * c + k] = t0 + c < nc ? float(double(dy[(t0 + c) * NOUT + k]) * scale) : 0.f;
+      }
+      __syncthreads();
+    }
+    // ---- stage dz: 16 threads a row, four features each
+#pragma unroll
+    for (int r = 0; r < BT / 16; ++r) {
+      const int c = (t >> 4) + 16 * r, q = t & 15;
+      const int64_t cc = t0 + c;
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (cc < nc) {
+        if (TOP) {
+#pragma unroll
+          for (int k = 0; k < NOUT; ++k) {
+            const float v = sdy[8 * c + k];
+            const __nv_bfloat16* wr = wo + k * W + 4 * q;
+            fma4(d, v, make_float4(__bfloat162float(wr[0]), __bfloat162float(wr[1]), __bfloat162float(wr[2]),
+                                   __bfloat162float(wr[3])));
+          }
+        } else {
+          const int32_t e1 = off[cc + 1];
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int32_t e = off[cc]; e < e1; ++e) {
+            const int32_t o = nb[e];
+            const float deg = float(off[o + 1] - off[o]);
+            const float4 v = *reinterpret_cast<const float4*>(dagg_in + int64_t(o) * W + 4 * q);
+            sum.x += v.x / deg, sum.y += v.y / deg, sum.z += v.z / deg, sum.w += v.w / deg;
+          }
+          d = *reinterpret_cast<const float4*>(dh_in + cc * W + 4 * q);
+          d.x += sum.x, d.y += sum.y, d.z += sum.z, d.w += sum.w;
+        }
+        const float4 zz = *reinterpret_cast<const float4*>(z + cc * W + 4 * q);
+        d.x *= gelu_grad(zz.x), d.y *= gelu_grad(zz.y), d.z *= gelu_grad(zz.z), d.w *= gelu_grad(zz.w);
+      }
+      *reinterpret_cast<float4*>(sdz + c * BZS + 4 * q) = d;
+    }
+    // ---- stage the layer's inputs as the forward GEMM used them
+    constexpr int CH = FIN / 8;  // 8-element chunks of one half row
+    for (int i = t; i < BT * 2 * CH; i += BTH) {
+      const int c = i / (2 * CH), q = i - 2 * CH * c;
+      const int64_t cc = t0 + c;
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = 0.f;
+      if (cc < nc) {
+        if (q < CH) {
+          Chunk8<TA> ch;
+          ch.load(h + cc * FIN + 8 * q);
+          ch.get(v);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[k] = as_input<TA>(v[k]);
+        } else {
+          Chunk8<__nv_bfloat16> ch;
+          ch.load(agg + cc * FIN + 8 * (q - CH));
+          ch.get(v);
+        }
+      }
+      float4* o = reinterpret_cast<float4*>(sa + c * NC + 8 * q);
+      o[0] = make_float4(v[0], v[1], v[2], v[3]);
+      o[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    __syncthreads();
+    // ---- weight gradient: g[r][.] += dz[c][4 jg + r] a[c][.], cells in order
+    if constexpr (NI == 8) {
+#pragma unroll 4
+      for (int c = 0; c < BT; ++c) {
+        const float4 d = *reinterpret_cast<const float4*>(sdz + c * BZS + 4 * jg);
+        const float4 a0 = *reinterpret_cast<const float4*>(sa + c * NC + 4 * ig);
+        const float4 a1 = *reinterpret_cast<const float4*>(sa + c * NC + 64 + 4 * ig);
+        const float dv[4] = {d.x, d.y, d.z, d.w};
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) g[r][k] = fmaf(dv[r], av[k], g[r][k]);
+      }
     } else {
-      for (int64_t c = c0; c < c1; ++c) s += dz[c * nout + j];
+#pragma unroll 4
+      for (int c = 0; c < BT; ++c) {
+        const float4 d = *reinterpret_cast<const float4*>(sdz + c * BZS + 4 * jg);
+        const float dv[4] = {d.x, d.y, d.z, d.w};
+        float av[NI];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) av[k] = sa[c * NC + ig + 16 * k];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int k = 0; k < NI; ++k) g[r][k] = fmaf(dv[r], av[k], g[r][k]);
+      }
     }
-    o[w] = s;
+#pragma unroll 4
+    for (int c = 16 * bq; c < 16 * bq + 16; ++c) {
+      gb += sdz[c * BZS + bj];
+      if (TOP) {
+        const float hv = t0 + c < nc ? __bfloat162float(hout[(t0 + c) * W + bj]) : 0.f;
+#pragma unroll
+        for (int k = 0; k < NOUT; ++k) go[k] = fmaf(sdy[8 * c + k], hv, go[k]);
+        if (bj < NOUT) gbo += sdy[8 * c + bj];
+      }
+    }
+    // ---- dh_out = dz Ws, dagg_out = dz Wn: warp w cells w + 8 k, lane four columns
+    if constexpr (DENSE) {
+      float4 acc[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+      for (int j = 0; j < W; j += 4) {
+        float4 d[8], w4;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) d[k] = *reinterpret_cast<const float4*>(sdz + (warp + 8 * k) * BZS + j);
+        w4 = *reinterpret_cast<const float4*>(sw + j * NC + 4 * lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].x, w4);
+        w4 = *reinterpret_cast<const float4*>(sw + (j + 1) * NC + 4 * lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].y, w4);
+        w4 = *reinterpret_cast<const float4*>(sw + (j + 2) * NC + 4 * lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].z, w4);
+        w4 = *reinterpret_cast<const float4*>(sw + (j + 3) * NC + 4 * lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].w, w4);
+      }
+      float* o = lane < 16 ? dh_out + 4 * lane : dagg_out + 4 * (lane - 16);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int64_t cc = t0 + warp + 8 * k;
+        if (cc < nc) *reinterpret_cast<float4*>(o + cc * W) = acc[k];
+      }
+    }
   }
-}
-// g[wofs + j*fin + i] (and g[bofs + j] when bofs >= 0) = sum over blocks
-__global__ void k_wgrad_reduce(int nblk, int nout, int fin, const float* __restrict__ part,
-                               float* __restrict__ g, int64_t wofs, int64_t bofs) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= nout * (fin + 1)) return;
-  const int j = w / (fin + 1), i = w % (fin + 1);
-  double s = 0;
-  for (int b = 0; b < nblk; ++b) s += part[int64_t(b) * nout * (fin + 1) + w];
-  if (i < fin)
-    g[wofs + j * fin + i] = float(s);
-  else if (bofs >= 0)
-    g[bofs + j] = float(s);
-}
-
-// dh[c][i] = sum_j W[j][i] dz[c][j]   (W: nout x fin, bf16)
-__global__ void __launch_bounds__(GT) k_back_dense(int64_t nc, int nout, int fin,
-                                                   const __nv_bfloat16* __restrict__ w,
-                                                   const float* __restrict__ dz,
-                                                   float* __restrict__ dh) {
-  __shared__ float sw[W * W];
-  for (int i = threadIdx.x; i < nout * fin; i += GT) sw[i] = __bfloat162float(w[i]);
+  // ---- the CTA's partials
+  float* o = part + int64_t(blockIdx.x) * back_part(FIN, TOP);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int k = 0; k < NI; ++k)
+      o[(4 * jg + r) * NC + (NI == 8 ? (k < 4 ? 4 * ig + k : 64 + 4 * ig + k - 4) : ig + 16 * k)] = g[r][k];
+  constexpr int RS = W + NOUT * W + 8;
   __syncthreads();
-  const int64_t c = int64_t(blockIdx.x) * GT + threadIdx.x;
-  if (c >= nc) return;
-  for (int i0 = 0; i0 < fin; i0 += 16) {
-    float acc[16];
+  sred[bq * RS + bj] = gb;
+  if (TOP) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    for (int j = 0; j < nout; ++j) {
-      const float d = dz[c * nout + j];
+    for (int k = 0; k < NOUT; ++k) sred[bq * RS + W + k * W + bj] = go[k];
+    if (bj < NOUT) sred[bq * RS + W + NOUT * W + bj] = gbo;
+  }
+  __syncthreads();
+  for (int i = t; i < W + (TOP ? NOUT * W + NOUT : 0); i += BTH) {
+    float v = 0.f;
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (i0 + i < fin) acc[i] += sw[j * fin + i0 + i] * d;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (i0 + i < fin) dh[c * fin + i0 + i] = acc[i];
+    for (int q = 0; q < 4; ++q) v += sred[q * RS + i];
+    o[W * NC + i] = v;
   }
 }
 
-// dh[n] += sum_{c in N(n)} dagg[c] / deg(c)  (the graph is symmetric)
-__global__ void k_back_aggregate(int64_t nc, int fin, const int32_t* __restrict__ off,
-                                 const int32_t* __restrict__ nb, const float* __restrict__ dagg,
-                                 float* __restrict__ dh) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nc * fin) return;
-  const int64_t n = i / fin;
-  const int k = int(i % fin);
-  float s = 0.f;
-  for (int32_t e = off[n]; e < off[n + 1]; ++e) {
-    const int32_t c = nb[e];
-    const int32_t deg = off[c + 1] - off[c];
-    s += dagg[int64_t(c) * fin + k] / float(deg);
+// Cells per CTA of k_back_layer on a device that holds `slots` of its CTAs at
+// once: whole tiles, at most RB, in the fewest rounds of CTAs times tiles
+// (a CTA's start and partial cost about a fifth of a tile).  1,296 cells
+// take 64 and spread over the device (a training step of 0.13 ms against
+// 0.24 with RB); 82,944 take 64 in five rounds, where RB would leave a
+// second round of 28 CTAs; large graphs take RB and write few partials.
+constexpr int64_t BACK_SMALL = 8;  // below RB only where that is at most this many rounds
+inline int back_cells(int64_t nc, int64_t slots) {
+  const int64_t nt = (nc + BT - 1) / BT;
+  int best = RB / BT;
+  double cost = 1e300;
+  for (int k = RB / BT; k >= 1; --k) {
+    const int64_t rounds = ((nt + k - 1) / k + slots - 1) / slots;
+    if (k < RB / BT && rounds > BACK_SMALL) break;
+    if (rounds * (k + 0.2) < cost) cost = rounds * (k + 0.2), best = k;
   }
-  dh[i] += s;
+  return best * BT;
 }
 
-// dz = dh * GELU'(z)
-__global__ void k_back_gelu(int64_t n, const float* __restrict__ dh, const float* __restrict__ z,
-                            float* __restrict__ dz) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) dz[i] = dh[i] * gelu_grad(z[i]);
+// the parameters' gradients from the CTAs' partials (np values each): a warp
+// per 32 values and every BRW-th CTA, then the warps, in a fixed order
+constexpr int BRW = 8;
+struct BackDst {
+  int64_t ws, wn, b, wo, bo;
+};
+__global__ void __launch_bounds__(32 * BRW) k_back_reduce(int nblk, int np, int fin, const float* __restrict__ part,
+                                                         float* __restrict__ g, BackDst D) {
+  __shared__ double sh[BRW][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = blockIdx.x * 32 + lane;
+  double s = 0;
+  if (w < np) {
+#pragma unroll 4
+    for (int b = warp; b < nblk; b += BRW) s += double(part[int64_t(b) * np + w]);
+  }
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || w >= np) return;
+#pragma unroll
+  for (int k = 1; k < BRW; ++k) s += sh[k][lane];
+  const int n0 = W * 2 * fin, n1 = n0 + W, n2 = n1 + NOUT * W;
+  int64_t at;
+  if (w < n0) {
+    const int j = w / (2 * fin), i = w - 2 * fin * j;
+    at = i < fin ? D.ws + j * fin + i : D.wn + j * fin + i - fin;
+  } else if (w < n1) {
+    at = D.b + w - n0;
+  } else {
+    at = w < n2 ? D.wo + w - n1 : D.bo + w - n2;
+  }
+  g[at] = float(s);
 }
 
 __global__ void k_adam(int64_t n, float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
@@ -1203,44 +1395,6 @@ int take_error(fpsi_gnn* m) {
   return FPSI_E_TIMEOUT;
 }
 
-// loss over the batch and full gradient into m->d_g; loss_out (device) [2]
-int backward(fpsi_gnn* m, const Graph& G, const float* feat, const float* target, const float* mask,
-             uint64_t seed, uint64_t thr, double* loss_out) {
-  cudaStream_t s = m->stream;
-  const int64_t nc = G.nc;
-  const int nblk = int(nb_(nc, GT));
-  float* dy = m->d_dz;  // [nc][5] fits in the [nc][64] buffer
-  k_loss<<<nblk, GT, 0, s>>>(nc, m->d_y, target, seed, thr, mask, dy, m->d_lpart);
-  k_loss_final<<<1, 256, 0, s>>>(m->d_lpart, nblk, loss_out);
-  k_scale<<<nb_(nc * NOUT, 256), 256, 0, s>>>(nc * NOUT, dy, loss_out);
-  const int rb = int(nb_(nc, RB));
-  // head
-  k_wgrad_partial<__nv_bfloat16><<<rb, 256, 0, s>>>(nc, NOUT, W, dy, m->d_h[NLAYER], m->d_part);
-  k_wgrad_reduce<<<nb_(NOUT * (W + 1), 256), 256, 0, s>>>(rb, NOUT, W, m->d_part, m->d_g, m->L.wo, m->L.bo);
-  k_back_dense<<<nb_(nc, GT), GT, 0, s>>>(nc, NOUT, W, m->d_wb + m->L.wo, dy, m->d_dh);
-  for (int l = NLAYER - 1; l >= 0; --l) {
-    const int fin = m->L.fan_in[l];
-    k_back_gelu<<<nb_(nc * W, 256), 256, 0, s>>>(nc * W, m->d_dh, m->d_z[l], m->d_dz);
-    if (l == 0)
-      k_wgrad_partial<float><<<rb, 256, 0, s>>>(nc, W, fin, m->d_dz, feat, m->d_part);
-    else
-      k_wgrad_partial<__nv_bfloat16><<<rb, 256, 0, s>>>(nc, W, fin, m->d_dz, m->d_h[l], m->d_part);
-    k_wgrad_reduce<<<nb_(W * (fin + 1), 256), 256, 0, s>>>(rb, W, fin, m->d_part, m->d_g, m->L.ws[l],
-                                                          m->L.b[l]);
-    k_wgrad_partial<__nv_bfloat16><<<rb, 256, 0, s>>>(nc, W, fin, m->d_dz, m->d_agg[l], m->d_part);
-    k_wgrad_reduce<<<nb_(W * (fin + 1), 256), 256, 0, s>>>(rb, W, fin, m->d_part, m->d_g, m->L.wn[l], -1);
-    if (l > 0) {
-      // dh_in = Ws^T dz + scatter(Wn^T dz)
-      k_back_dense<<<nb_(nc, GT), GT, 0, s>>>(nc, W, fin, m->d_wb + m->L.wn[l], m->d_dz, m->d_dagg);
-      k_back_dense<<<nb_(nc, GT), GT, 0, s>>>(nc, W, fin, m->d_wb + m->L.ws[l], m->d_dz, m->d_dh2);
-      k_back_aggregate<<<nb_(nc * fin, 256), 256, 0, s>>>(nc, fin, G.off, G.nb, m->d_dagg, m->d_dh2);
-      std::swap(m->d_dh, m->d_dh2);
-    }
-  }
-  FPSI_CUDA_TRY(cudaGetLastError());
-  return FPSI_OK;
-}
-
 template <class T>
 int galloc(T** p, size_t n) {
   if (cudaMalloc((void**)p, (n ? n : 1) * sizeof(T)) != cudaSuccess) {
@@ -1251,11 +1405,60 @@ int galloc(T** p, size_t n) {
   return FPSI_OK;
 }
 
+// loss over the batch and full gradient into m->d_g; loss_out (device) [2]
+int backward(fpsi_gnn* m, const Graph& G, const float* feat, const float* target, const float* mask,
+             uint64_t seed, uint64_t thr, double* loss_out) {
+  cudaStream_t s = m->stream;
+  const int64_t nc = G.nc;
+  const int nblk = int(nb_(nc, GT));
+  float* dy = m->d_dz;  // [nc][5] fits in the [nc][64] buffer; read by the last layer only
+  k_loss<<<nblk, GT, 0, s>>>(nc, m->d_y, target, seed, thr, mask, dy, m->d_lpart);
+  k_loss_final<<<1, 256, 0, s>>>(m->d_lpart, nblk, loss_out);
+  const int rbc = back_cells(nc, 2 * m->nsm);
+  const unsigned rb = nb_(nc, rbc);
+  if (int64_t(rb) > m->part_cap) {
+    FPSI_CUDA_TRY(cudaStreamSynchronize(s));
+    if (m->d_part) cudaFree(m->d_part);
+    m->part_cap = 0;
+    const int rc = galloc(&m->d_part, size_t(rb) * back_part(W, true));
+    if (rc) return rc;
+    m->part_cap = rb;
+  }
+  // a layer reads the two parts of dh that the layer above wrote and writes
+  // its own into the other pair of buffers
+  float *dh = m->d_dh, *dagg = m->d_dz, *dh2 = m->d_dh2, *dagg2 = m->d_dagg;
+  for (int l = NLAYER - 1; l >= 0; --l) {
+    const int fin = m->L.fan_in[l];
+    const bool top = l == NLAYER - 1, dense = l > 0;
+    const size_t smem = size_t(back_smem(fin, dense).total) * sizeof(float);
+    const __nv_bfloat16 *ws = m->d_wb + m->L.ws[l], *wn = m->d_wb + m->L.wn[l], *wo = m->d_wb + m->L.wo;
+    if (top)
+      k_back_layer<W, true, true, __nv_bfloat16><<<rb, BTH, smem, s>>>(
+          nc, rbc, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, nullptr, nullptr, dy, loss_out, wo,
+          m->d_h[NLAYER], dh2, dagg2, m->d_part);
+    else if (dense)
+      k_back_layer<W, false, true, __nv_bfloat16><<<rb, BTH, smem, s>>>(
+          nc, rbc, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr,
+          nullptr, dh2, dagg2, m->d_part);
+    else
+      k_back_layer<NIN, false, false, float><<<rb, BTH, smem, s>>>(
+          nc, rbc, G.off, G.nb, m->d_z[l], feat, m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr, nullptr,
+          nullptr, nullptr, m->d_part);
+    const int np = back_part(fin, top);
+    k_back_reduce<<<nb_(np, 32), 32 * BRW, 0, s>>>(int(rb), np, fin, m->d_part, m->d_g,
+                                                  BackDst{m->L.ws[l], m->L.wn[l], m->L.b[l], m->L.wo, m->L.bo});
+    std::swap(dh, dh2);
+    std::swap(dagg, dagg2);
+  }
+  FPSI_CUDA_TRY(cudaGetLastError());
+  return FPSI_OK;
+}
+
 void free_activations(fpsi_gnn* m) {
-  void* ps[] = {m->d_y, m->d_dh, m->d_dh2, m->d_dz, m->d_dagg, m->d_part, m->d_lpart};
+  void* ps[] = {m->d_y, m->d_dh, m->d_dh2, m->d_dz, m->d_dagg, m->d_lpart};
   for (void* p : ps)
     if (p) cudaFree(p);
-  m->d_y = m->d_dh = m->d_dh2 = m->d_dz = m->d_dagg = m->d_part = nullptr;
+  m->d_y = m->d_dh = m->d_dh2 = m->d_dz = m->d_dagg = nullptr;
   m->d_lpart = nullptr;
   for (int l = 0; l <= NLAYER; ++l) {
     if (m->d_h[l]) cudaFree(m->d_h[l]);
@@ -1288,7 +1491,6 @@ int ensure_capacity(fpsi_gnn* m, int64_t nc) {
   G(galloc(&m->d_dh2, nc * W));
   G(galloc(&m->d_dz, nc * W));
   G(galloc(&m->d_dagg, nc * W));
-  G(galloc(&m->d_part, ((nc + RB - 1) / RB) * W * (W + 1)));
   G(galloc(&m->d_lpart, ((nc + GT - 1) / GT) * 10 + 16));
 #undef G
   if (rc) {
@@ -1374,6 +1576,15 @@ int fpsi_gnn_create(fpsi_gnn** out, uint64_t seed) {
                                    int(tc_smem(W).total)) != cudaSuccess ||
               cudaFuncSetAttribute(k_layer_tc<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(tc_smem(W).total)) != cudaSuccess ||
+              cudaFuncSetAttribute(k_back_layer<W, true, true, __nv_bfloat16>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(back_smem(W, true).total * sizeof(float))) != cudaSuccess ||
+              cudaFuncSetAttribute(k_back_layer<W, false, true, __nv_bfloat16>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(back_smem(W, true).total * sizeof(float))) != cudaSuccess ||
+              cudaFuncSetAttribute(k_back_layer<NIN, false, false, float>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(back_smem(NIN, false).total * sizeof(float))) != cudaSuccess ||
               cudaFuncSetAttribute(k_layer_ws<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(ws_smem(W).total)) != cudaSuccess ||
               cudaFuncSetAttribute(k_layer_ws<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1424,7 +1635,7 @@ int fpsi_gnn_destroy(fpsi_gnn* m) {
   if (!m) return FPSI_OK;
   fpsi_gnn_clear_snapshots(m);
   free_activations(m);
-  void* ps[] = {m->d_w, m->d_m, m->d_v, m->d_g, m->d_wb, m->d_err, m->d_fac};
+  void* ps[] = {m->d_w, m->d_m, m->d_v, m->d_g, m->d_wb, m->d_err, m->d_fac, m->d_part};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (m->stream) cudaStreamDestroy(m->stream);
