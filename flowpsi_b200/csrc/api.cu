@@ -293,6 +293,22 @@ void unpermute_cells(const fpsi_ctx* x, const T* dev_order, int w, T* caller) {
   }
 }
 
+// per-cell device rows (w <= 5 values) into a caller-order host array, and
+// back: permuted on the device through the staging buffer
+int rows_down(fpsi_ctx* x, int w, const int32_t* map, const void* src, int bytes, double* out) {
+  int rc = fpsi::launch_rows_out(x, w, map, src, bytes, x->d_stage);
+  if (rc) return rc;
+  FPSI_CUDA_TRY(cudaMemcpyAsync(out, x->d_stage, size_t(x->H.nc) * w * sizeof(double), cudaMemcpyDeviceToHost,
+                                x->stream));
+  return sync(x);
+}
+int rows_up(fpsi_ctx* x, int w, const int32_t* map, const double* in, void* dst, int bytes) {
+  FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage, in, size_t(x->H.nc) * w * sizeof(double), cudaMemcpyHostToDevice,
+                                x->stream));
+  const int rc = fpsi::launch_rows_in(x, w, map, x->d_stage, dst, bytes);
+  return rc ? rc : sync(x);
+}
+
 }  // namespace
 
 extern "C" {
@@ -613,30 +629,20 @@ int fpsi_get_lines(fpsi_ctx* x, int32_t* line_of_cell, int32_t* position, int32_
 
 int fpsi_set_eddy_viscosity(fpsi_ctx* x, const double* tmu) {
   if (!x || !tmu) return FPSI_E_INVALID;
-  std::vector<double> t(x->H.nc);
-  for (int64_t i = 0; i < x->H.nc; ++i) t[i] = tmu[x->H.perm[i]];
-  FPSI_CUDA_TRY(cudaMemcpy(x->d_tmu, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+  const int rc = rows_up(x, 1, nullptr, tmu, x->d_tmu, 8);
+  if (rc) return rc;
   x->have_resid = x->have_asm = x->have_dq = false;
   return FPSI_OK;
 }
 
 // ---- Spalart-Allmaras nu~ -------------------------------------------------
-static int sa_down(fpsi_ctx* x, const double* d, double* out) {
-  std::vector<double> h(x->H.nc);
-  FPSI_CUDA_TRY(cudaMemcpyAsync(h.data(), d, h.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                                x->stream));
-  int rc = sync(x);
-  if (rc) return rc;
-  for (int64_t i = 0; i < x->H.nc; ++i) out[x->H.perm[i]] = h[i];
-  return FPSI_OK;
-}
+static int sa_down(fpsi_ctx* x, const double* d, double* out) { return rows_down(x, 1, nullptr, d, 8, out); }
 
 int fpsi_set_nutilde(fpsi_ctx* x, const double* nut) {
   if (!x || !nut) return FPSI_E_INVALID;
   if (!x->d_nut) return FPSI_E_STATE;
-  std::vector<double> t(x->H.nc);
-  for (int64_t i = 0; i < x->H.nc; ++i) t[i] = nut[x->H.perm[i]];
-  FPSI_CUDA_TRY(cudaMemcpy(x->d_nut, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+  const int rc = rows_up(x, 1, nullptr, nut, x->d_nut, 8);
+  if (rc) return rc;
   x->have_resid = x->have_asm = x->have_dq = x->have_sa = x->have_sa_dq = false;
   return FPSI_OK;
 }
@@ -759,14 +765,7 @@ int fpsi_residual(fpsi_ctx* x, double* src, fpsi_resid* norms) {
   if (rc) return rc;
   FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid, x->d_resid, fpsi::NREC * sizeof(double),
                                 cudaMemcpyDeviceToHost, x->stream));
-  std::vector<double> s;
-  if (src) {
-    s.resize(5 * x->H.nc);
-    FPSI_CUDA_TRY(cudaMemcpyAsync(s.data(), x->d_src, s.size() * sizeof(double),
-                                  cudaMemcpyDeviceToHost, x->stream));
-  }
-  if ((rc = sync(x))) return rc;
-  if (src) unpermute_cells(x, s.data(), 5, src);
+  if ((rc = src ? rows_down(x, 5, nullptr, x->d_src, 8, src) : sync(x))) return rc;
   if (norms) fill_norms(x, x->h_resid, norms);
   x->have_resid = true;
   x->have_asm = x->have_dq = x->x_preset = false;
@@ -801,10 +800,7 @@ int fpsi_get_reconstruction(fpsi_ctx* x, double* grad, double* limiter) {
 int fpsi_get_dtau(fpsi_ctx* x, double* dtau) {
   if (!x || !dtau) return FPSI_E_INVALID;
   if (!x->have_resid) return FPSI_E_STATE;
-  std::vector<double> d(x->H.nc);
-  FPSI_CUDA_TRY(cudaMemcpy(d.data(), x->d_dtau, d.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  unpermute_cells(x, d.data(), 1, dtau);
-  return FPSI_OK;
+  return rows_down(x, 1, nullptr, x->d_dtau, 8, dtau);
 }
 
 static int finish_assemble(fpsi_ctx* x) {
@@ -901,67 +897,14 @@ int fpsi_get_blocks(fpsi_ctx* x, void* D, void* fjp, void* fjm, void* B) {
   return FPSI_OK;
 }
 
+// the iterate: colour order, or line order (whose padding rows stay as they are)
 static int upload_x(fpsi_ctx* x, const double* x0) {
-  const int64_t nc = x->H.nc;
-  if (is_lsgs(x)) {
-    const size_t nt = size_t(x->LY.nrows) * 32;
-    std::vector<double> v(5 * nt, 0.0);
-    for (int64_t i = 0; i < nc; ++i)
-      for (int k = 0; k < 5; ++k)
-        v[5 * int64_t(x->LY.t_of[i]) + k] = x0[5 * int64_t(x->H.perm[i]) + k];
-    if (x->x_bytes == 8 && x->P.precision != FPSI_PREC_MIXED) {
-      FPSI_CUDA_TRY(cudaMemcpy(x->d_lx, v.data(), v.size() * 8, cudaMemcpyHostToDevice));
-    } else {
-      std::vector<float> f(v.begin(), v.end());
-      FPSI_CUDA_TRY(cudaMemcpy(x->d_lx, f.data(), f.size() * 4, cudaMemcpyHostToDevice));
-    }
-    return FPSI_OK;
-  }
-  if (x->x_bytes == 8) {
-    std::vector<double> v(5 * nc);
-    for (int64_t i = 0; i < nc; ++i)
-      for (int k = 0; k < 5; ++k)
-        v[5 * int64_t(x->H.ci_of[i]) + k] = x0[5 * int64_t(x->H.perm[i]) + k];
-    FPSI_CUDA_TRY(cudaMemcpy(x->d_x, v.data(), v.size() * 8, cudaMemcpyHostToDevice));
-  } else {
-    std::vector<float> v(5 * nc);
-    for (int64_t i = 0; i < nc; ++i)
-      for (int k = 0; k < 5; ++k)
-        v[5 * int64_t(x->H.ci_of[i]) + k] = float(x0[5 * int64_t(x->H.perm[i]) + k]);
-    FPSI_CUDA_TRY(cudaMemcpy(x->d_x, v.data(), v.size() * 4, cudaMemcpyHostToDevice));
-  }
-  return FPSI_OK;
+  return is_lsgs(x) ? rows_up(x, 5, x->d_lt, x0, x->d_lx, x->x_bytes) : rows_up(x, 5, x->d_ci, x0, x->d_x, x->x_bytes);
 }
 
 static int download_x(fpsi_ctx* x, double* dq) {
-  const int64_t nc = x->H.nc;
-  if (is_lsgs(x)) {
-    const size_t nt = size_t(x->LY.nrows) * 32;
-    std::vector<double> v(5 * nt);
-    if (x->P.precision != FPSI_PREC_MIXED) {
-      FPSI_CUDA_TRY(cudaMemcpy(v.data(), x->d_lx, v.size() * 8, cudaMemcpyDeviceToHost));
-    } else {
-      std::vector<float> f(5 * nt);
-      FPSI_CUDA_TRY(cudaMemcpy(f.data(), x->d_lx, f.size() * 4, cudaMemcpyDeviceToHost));
-      for (size_t i = 0; i < f.size(); ++i) v[i] = f[i];
-    }
-    for (int64_t i = 0; i < nc; ++i)
-      for (int k = 0; k < 5; ++k)
-        dq[5 * int64_t(x->H.perm[i]) + k] = v[5 * int64_t(x->LY.t_of[i]) + k];
-    return FPSI_OK;
-  }
-  std::vector<double> v(5 * nc);
-  if (x->x_bytes == 8) {
-    FPSI_CUDA_TRY(cudaMemcpy(v.data(), x->d_x, v.size() * 8, cudaMemcpyDeviceToHost));
-  } else {
-    std::vector<float> f(5 * nc);
-    FPSI_CUDA_TRY(cudaMemcpy(f.data(), x->d_x, f.size() * 4, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < f.size(); ++i) v[i] = f[i];
-  }
-  for (int64_t i = 0; i < nc; ++i)
-    for (int k = 0; k < 5; ++k)
-      dq[5 * int64_t(x->H.perm[i]) + k] = v[5 * int64_t(x->H.ci_of[i]) + k];
-  return FPSI_OK;
+  return is_lsgs(x) ? rows_down(x, 5, x->d_lt, x->d_lx, x->x_bytes, dq)
+                    : rows_down(x, 5, x->d_ci, x->d_x, x->x_bytes, dq);
 }
 
 int fpsi_linear_solve(fpsi_ctx* x, const double* x0, double* dq, fpsi_lsinfo* info) {

@@ -1711,12 +1711,14 @@ static int make_features(fpsi_gnn* m, fpsi_ctx* x, float* feat, float* xj, float
   return FPSI_OK;
 }
 
-__global__ void k_target(int64_t nc, const double* __restrict__ dq_rcm, const float* __restrict__ xj,
-                         const float* __restrict__ scl, float* __restrict__ t) {
+// training targets (dq - x_J) / xs; row: where dq keeps cell c (null: at c)
+__global__ void k_target(int64_t nc, const double* __restrict__ dq, const int32_t* __restrict__ row,
+                         const float* __restrict__ xj, const float* __restrict__ scl, float* __restrict__ t) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= nc * 5) return;
   const int k = int(i % 5);
-  t[i] = float((dq_rcm[i] - double(xj[i])) / double(scl[k]));
+  const double d = dq[row ? 5 * int64_t(row[i / 5]) + k : i];
+  t[i] = float((d - double(xj[i])) / double(scl[k]));
 }
 
 int fpsi_gnn_add_snapshot(fpsi_gnn* m, fpsi_ctx* x, const double* dq) {
@@ -1732,29 +1734,23 @@ int fpsi_gnn_add_snapshot(fpsi_gnn* m, fpsi_ctx* x, const double* dq) {
   if (!rc) rc = galloc(&s.target, nc * 5);
   if (!rc) rc = galloc(&s.xj, nc * 5);
   if (!rc) rc = make_features(m, x, s.feat, s.xj, s.rs, s.xs);
-  double* dd = nullptr;
-  if (!rc) rc = galloc(&dd, nc * 5);
   if (rc) {
     free_snapshot(s);
     return rc;
   }
   s.nc = nc;
   s.perm = x->H.perm;
-  // target in RCM order
-  std::vector<double> d(nc * 5);
-  for (int64_t i = 0; i < nc; ++i)
-    for (int k = 0; k < 5; ++k) d[5 * i + k] = dq[5 * int64_t(s.perm[i]) + k];
+  double* dd = x->d_stage;  // dq in the caller's order; no call on x is in flight
   float* dscl = reinterpret_cast<float*>(m->d_lpart);
   bool ok = cudaMemcpyAsync(s.d_off, G.off, (nc + 1) * 4, cudaMemcpyDeviceToDevice, m->stream) == cudaSuccess &&
             (x->cnb_n == 0 || cudaMemcpyAsync(s.d_nb, G.nb, x->cnb_n * 4, cudaMemcpyDeviceToDevice,
                                               m->stream) == cudaSuccess) &&
-            cudaMemcpyAsync(dd, d.data(), d.size() * 8, cudaMemcpyHostToDevice, m->stream) == cudaSuccess &&
+            cudaMemcpyAsync(dd, dq, size_t(nc) * 5 * 8, cudaMemcpyHostToDevice, m->stream) == cudaSuccess &&
             cudaMemcpyAsync(dscl, s.xs, 5 * sizeof(float), cudaMemcpyHostToDevice, m->stream) == cudaSuccess;
   if (ok) {
-    k_target<<<nb_(nc * 5, 256), 256, 0, m->stream>>>(nc, dd, s.xj, dscl, s.target);
+    k_target<<<nb_(nc * 5, 256), 256, 0, m->stream>>>(nc, dd, x->d_perm, s.xj, dscl, s.target);
     ok = cudaStreamSynchronize(m->stream) == cudaSuccess;
   }
-  cudaFree(dd);
   if (!ok) {
     free_snapshot(s);
     fpsi::set_error("learned start: snapshot upload failed");
@@ -1862,7 +1858,7 @@ int fpsi_gnn_add_snapshot_region(fpsi_gnn* m, fpsi_ctx* x, const double* dq, con
   if (ok) {
     k_gather_rows<<<nb_(ns * NIN, 256), 256, 0, st>>>(ns, didx, NIN, ffull, s.feat);
     k_gather_rows<<<nb_(ns * 5, 256), 256, 0, st>>>(ns, didx, 5, xfull, s.xj);
-    k_target<<<nb_(ns * 5, 256), 256, 0, st>>>(ns, dd, s.xj, dscl, s.target);
+    k_target<<<nb_(ns * 5, 256), 256, 0, st>>>(ns, dd, nullptr, s.xj, dscl, s.target);
     ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
   }
   cudaFree(didx);
@@ -2034,10 +2030,11 @@ __global__ void k_features_bf16(int64_t nc, const double* __restrict__ src, cons
 }
 
 // x0 = x_J + xs * d into ctx's colour-order iterate, which holds x_J (the
-// next linear solve starts from it); x0_out (RCM order) optional
+// next linear solve starts from it); x0 (caller order, by perm) optional
 template <class TX>
 __global__ void k_apply_start(int64_t nc, const float* __restrict__ y, const float* __restrict__ fac,
-                              const int32_t* __restrict__ ci, TX* __restrict__ x, double* __restrict__ x0) {
+                              const int32_t* __restrict__ ci, const int32_t* __restrict__ perm, TX* __restrict__ x,
+                              double* __restrict__ x0) {
   const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= nc) return;
   const int64_t i = ci[c];
@@ -2045,7 +2042,7 @@ __global__ void k_apply_start(int64_t nc, const float* __restrict__ y, const flo
     const float xj = float(x[5 * i + k]);
     const double v = double(xj) + double(fac[5 + k]) * double(y[c * 5 + k]);
     x[5 * i + k] = TX(v);
-    if (x0) x0[5 * c + k] = v;
+    if (x0) x0[5 * int64_t(perm[c]) + k] = v;
   }
 }
 
@@ -2070,27 +2067,19 @@ extern "C" {
 int fpsi_gnn_predict(fpsi_gnn* m, fpsi_ctx* x, double* x0) {
   if (!m || !x) return FPSI_E_INVALID;
   const int64_t nc = x->H.nc;
-  double* dx0 = nullptr;
-  int rc = FPSI_OK;
-  if (x0 && (rc = galloc(&dx0, nc * 5))) return rc;
-  rc = fpsi::gnn_predict_launch(m, x, dx0);
+  int rc = fpsi::gnn_predict_launch(m, x, x0 ? x->d_stage : nullptr);
+  if (!rc && x0 &&
+      cudaMemcpyAsync(x0, x->d_stage, size_t(nc) * 5 * sizeof(double), cudaMemcpyDeviceToHost, x->stream) != cudaSuccess)
+    rc = FPSI_E_CUDA;
   if (!rc && cudaStreamSynchronize(x->stream) != cudaSuccess) rc = FPSI_E_CUDA;
-  if (!rc) rc = take_error(m);
-  if (!rc && x0) {
-    std::vector<double> h(nc * 5);
-    if (cudaMemcpy(h.data(), dx0, h.size() * 8, cudaMemcpyDeviceToHost) != cudaSuccess) rc = FPSI_E_CUDA;
-    for (int64_t i = 0; !rc && i < nc; ++i)
-      for (int k = 0; k < 5; ++k) x0[5 * int64_t(x->H.perm[i]) + k] = h[5 * i + k];
-  }
-  cudaFree(dx0);
-  return rc;
+  return rc ? rc : take_error(m);
 }
 
 }  // extern "C"
 namespace fpsi {
 // Inference queued on the context's stream with no host synchronisation:
 // the Jacobi start, the features, the layers and the start written into the
-// iterate (and, with dx0, a copy in RCM order).  The model's error bits
+// iterate (and, with dx0, a copy in the caller's order).  The model's error bits
 // (gnn_error_bits) are left for the caller to read.  jacobi_in_iterate: the
 // iterate already holds D^-1 B (an SGS assembly has just written it).
 int32_t* gnn_error_bits(fpsi_gnn* m) { return m->d_err; }
@@ -2129,9 +2118,9 @@ int gnn_predict_launch(fpsi_gnn* m, fpsi_ctx* x, double* dx0, bool jacobi_in_ite
     launch_features16<float, double>(m, x, feat16, s);
   if ((rc = forward(m, G, nullptr, false, feat16, s))) return rc;
   if (x->P.precision == FPSI_PREC_MIXED)
-    k_apply_start<float><<<nb_(nc, 256), 256, 0, s>>>(nc, m->d_y, m->d_fac, x->d_ci, (float*)x->d_x, dx0);
+    k_apply_start<float><<<nb_(nc, 256), 256, 0, s>>>(nc, m->d_y, m->d_fac, x->d_ci, x->d_perm, (float*)x->d_x, dx0);
   else
-    k_apply_start<double><<<nb_(nc, 256), 256, 0, s>>>(nc, m->d_y, m->d_fac, x->d_ci, (double*)x->d_x, dx0);
+    k_apply_start<double><<<nb_(nc, 256), 256, 0, s>>>(nc, m->d_y, m->d_fac, x->d_ci, x->d_perm, (double*)x->d_x, dx0);
   FPSI_CUDA_TRY(cudaGetLastError());
   x->x_preset = true;
   return FPSI_OK;

@@ -34,6 +34,12 @@ int launch_update(fpsi_ctx* x, const double* guard, const int32_t* flag0 = nullp
 // caller-order staging buffer <-> device state (in = staging -> q)
 int launch_state(fpsi_ctx* x, bool in);
 
+// rows of w values per cell: device order (map: RCM cell -> row, null RCM
+// order; values of 4 or 8 bytes) to or from a caller-order array of doubles
+// on the device
+int launch_rows_out(fpsi_ctx* x, int w, const int32_t* map, const void* src, int bytes, double* caller);
+int launch_rows_in(fpsi_ctx* x, int w, const int32_t* map, const double* caller, void* dst, int bytes);
+
 int launch_batch_flux(int kind, int64_t n, const double* qL, const double* qR, const double* an,
                       const double* area, double pamb, double Rt, double gamma, double us_n,
                       double eta, double* F, cudaStream_t s);
