@@ -169,7 +169,7 @@ int alloc_lsgs(fpsi_ctx* x) {
   if ((rc = upload(x, &x->d_lonbr, Y.onbr))) return rc;
   if ((rc = upload(x, &x->d_llen, Y.lane_len))) return rc;
   if ((rc = upload(x, &x->d_lrow0, Y.grp_row0))) return rc;
-  if ((rc = dalloc(x, (char**)&x->d_lD, nt * 25 * td))) return rc;
+  if ((rc = dalloc(x, (char**)&x->d_lD, nt * 30 * td))) return rc;  // the block and its pivots' reciprocals
   if ((rc = dalloc(x, (char**)&x->d_lL, nt * 25 * tb))) return rc;
   if ((rc = dalloc(x, (char**)&x->d_lU, nt * 25 * tb))) return rc;
   if ((rc = dalloc(x, (char**)&x->d_lF, nt * size_t(Y.mout) * 25 * tb))) return rc;
@@ -179,7 +179,11 @@ int alloc_lsgs(fpsi_ctx* x) {
   if ((rc = dalloc(x, (char**)&x->d_lxt, nt * 5 * tx))) return rc;
   if ((rc = dalloc(x, (char**)&x->d_lctl, 64))) return rc;
   if ((rc = dalloc(x, &x->d_lpart, (nt + 255) / 256 + 1))) return rc;
-  // padding cells must read as zero in the relaxation and the residual
+  // padding cells must read as zero in the relaxation and the residual, and
+  // couplings past a line's ends as zero in the line solves
+  FPSI_CUDA_TRY(cudaMemset(x->d_lD, 0, nt * 30 * td));
+  FPSI_CUDA_TRY(cudaMemset(x->d_lL, 0, nt * 25 * tb));
+  FPSI_CUDA_TRY(cudaMemset(x->d_lU, 0, nt * 25 * tb));
   FPSI_CUDA_TRY(cudaMemset(x->d_lx, 0, nt * 5 * tx));
   FPSI_CUDA_TRY(cudaMemset(x->d_lxt, 0, nt * 5 * tx));
   FPSI_CUDA_TRY(cudaMemset(x->d_lB, 0, nt * 5 * tb));

@@ -102,6 +102,7 @@ struct LineLayout {
   std::vector<int32_t> t_of;       // RCM cell -> t
   std::vector<int32_t> c_of_t;     // t -> RCM cell, -1 for padding
   std::vector<int8_t> role;        // per cf entry: 0 boundary, 1 prev, 2 next, 3+s outer slot s
+  int32_t max_len = 0;             // longest line
   int mout = 0;                    // outer slots per cell
   std::vector<int32_t> onbr;       // [(row*mout + s)*32 + lane]: t of the outer neighbour or -1
   std::vector<int32_t> line_of;    // RCM cell -> line id (caller-visible order)

@@ -19,6 +19,7 @@
 #include <array>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "fpsi_internal.h"
@@ -190,6 +191,7 @@ int build_lines(fpsi_ctx* x, const std::vector<std::vector<int32_t>>* given) {
   }
   Y.col_goff[ncol] = Y.ngroups;
   Y.nrows = row;
+  for (int32_t n : Y.grp_len) Y.max_len = std::max(Y.max_len, n);
   if (row * 32 >= (int64_t(1) << 31)) {
     set_error("lines: padded size too large");
     return FPSI_E_INVALID;
@@ -258,6 +260,70 @@ struct LsgsCtl {
   int32_t iter, done;
 };
 
+// A group row's blocks (D, L, U): entries 0..23 as six quads, [quad][32
+// lanes][4], then entry 24 [32 lanes]: a lane moves a block in seven accesses,
+// each contiguous over the warp.
+template <class T>
+struct alignas(4 * sizeof(T) < 16 ? 4 * sizeof(T) : 16) Quad {
+  T v[4];
+};
+template <class T>
+__device__ __forceinline__ void block_load(const T* row, int lane, T* b) {
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const Quad<T> w = *reinterpret_cast<const Quad<T>*>(row + (q * 32 + lane) * 4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[4 * q + i] = w.v[i];
+  }
+  b[24] = row[24 * 32 + lane];
+}
+template <class T>
+__device__ __forceinline__ void block_store(T* row, int lane, const T* b) {
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    Quad<T> w;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w.v[i] = b[4 * q + i];
+    *reinterpret_cast<Quad<T>*>(row + (q * 32 + lane) * 4) = w;
+  }
+  row[24 * 32 + lane] = b[24];
+}
+
+// A row of lD: the block, then (once factored) the reciprocals of its five
+// pivots, [5][32 lanes]; NaN for a pivot outside the range in which
+// quotient() is exact.
+constexpr int DROW = 30 * 32;
+
+// a / b from y = RN(1 / b): the reciprocal's own error is added back
+// (y + yl = 1 / b to twice the precision), so q is within one ulp of a / b,
+// and one correction by its exact remainder rounds it correctly (Markstein's
+// theorem: Computation of elementary functions on the IBM RISC System/6000
+// processor, IBM J. Res. Dev. 34, 1990).  Four dependent FMAs instead of a
+// division's sequence; the result is that of a / b bit for bit while b and a
+// are in the ranges of pivot_ok and tiny() (a zero keeps its value, not its
+// sign).
+template <class T>
+__device__ __forceinline__ T quotient(T a, T b, T y) {
+  const T yl = fma(-b, y, T(1)) * y;
+  const T q = fma(a, y, a * yl);
+  return fma(fma(-b, q, a), y, q);
+}
+// |b| in 2^-36 .. 2^28 (FP32), 2^-300 .. 2^300 (FP64)
+__device__ __forceinline__ bool pivot_ok(float b) { return fabsf(b) >= 0x1p-36f && fabsf(b) <= 0x1p28f; }
+__device__ __forceinline__ bool pivot_ok(double b) { return fabs(b) >= 0x1p-300 && fabs(b) <= 0x1p300; }
+// the smallest nonzero |a| so far, as a key (twice its bits, less one; zero
+// gives the largest key), and whether one below 2^-74 (2^-600) was among
+// them: there the remainder or the reciprocal's second part may underflow.
+// Above, an overflow ends in a NaN.
+__device__ __forceinline__ uint32_t key_min(uint32_t k, float a) { return min(k, 2u * __float_as_uint(a) - 1u); }
+__device__ __forceinline__ uint32_t key_min(uint32_t k, double a) {
+  return min(k, 2u * uint32_t(__double2hiint(a)) - 1u);
+}
+template <class T>
+__device__ __forceinline__ bool tiny(uint32_t k) {
+  return k < (sizeof(T) == 4 ? 2u * ((127u - 74u) << 23) : 2u * ((1023u - 600u) << 20)) - 1u;
+}
+
 // Gather the line-ordered system: raw diagonal block, in-line couplings
 // (row p to p-1 in L, to p+1 in U), outer couplings and B.  The coupling of
 // row c to neighbour n through face f is fjm_f when c = cl(f), -fjp_f when
@@ -276,8 +342,10 @@ __global__ void k_lsgs_scatter(int64_t nt, const int32_t* __restrict__ c_of_t,
   const int64_t c = c_of_t[t];
   if (c < 0) return;
   const int64_t r = t >> 5, lane = t & 31;
+  TD d[25];
 #pragma unroll
-  for (int e = 0; e < 25; ++e) lD[(r * 25 + e) * 32 + lane] = TD(__ldg(D + 25 * c + e));
+  for (int e = 0; e < 25; ++e) d[e] = TD(__ldg(D + 25 * c + e));
+  block_store<TD>(lD + r * DROW, int(lane), d);
 #pragma unroll
   for (int k = 0; k < 5; ++k) lB[(r * 5 + k) * 32 + lane] = TB(__ldg(src + 5 * c + k));
   for (int32_t e = cf_off[c]; e < cf_off[c + 1]; ++e) {
@@ -287,15 +355,16 @@ __global__ void k_lsgs_scatter(int64_t nt, const int32_t* __restrict__ c_of_t,
     const int64_t f = ent >> 1;
     const bool neg = ent & 1;
     const TB* A = neg ? fjp + 25 * f : fjm + 25 * f;
-    TB* o;
-    if (ro == 1)
-      o = lL + r * 25 * 32 + lane;
-    else if (ro == 2)
-      o = lU + r * 25 * 32 + lane;
-    else
-      o = lF + (r * V.mout + (ro - 3)) * 25 * 32 + lane;
+    TB b[25];
 #pragma unroll
-    for (int k = 0; k < 25; ++k) o[k * 32] = neg ? TB(-__ldg(A + k)) : __ldg(A + k);
+    for (int k = 0; k < 25; ++k) b[k] = neg ? TB(-__ldg(A + k)) : __ldg(A + k);
+    if (ro < 3) {
+      block_store<TB>((ro == 1 ? lL : lU) + r * 25 * 32, int(lane), b);
+    } else {
+      TB* o = lF + (r * V.mout + (ro - 3)) * 25 * 32 + lane;
+#pragma unroll
+      for (int k = 0; k < 25; ++k) o[k * 32] = b[k];
+    }
   }
 }
 
@@ -331,6 +400,22 @@ __device__ __forceinline__ void lu5_nopiv_solve(const T* A, TV* y) {
   }
 }
 
+// lu5_nopiv_solve with the pivots' reciprocals r[5]; key: of the dividends
+template <class T>
+__device__ __forceinline__ void lu5_recip_solve(const T* A, const T* r, T* y, uint32_t& key) {
+#pragma unroll
+  for (int i = 1; i < 5; ++i)
+#pragma unroll
+    for (int j = 0; j < i; ++j) y[i] -= A[5 * i + j] * y[j];
+#pragma unroll
+  for (int i = 4; i >= 0; --i) {
+#pragma unroll
+    for (int j = i + 1; j < 5; ++j) y[i] -= A[5 * i + j] * y[j];
+    key = key_min(key, y[i]);
+    y[i] = quotient<T>(y[i], A[6 * i], r[i]);
+  }
+}
+
 // block Thomas preprocessing (preprocessLine, linearSolverLSGS.loci:1465-1495):
 // D'_0 = D_0, D'_p = D_p - L_p D'_{p-1}^{-1} U_{p-1}; each D' factored in
 // place.  As in the reference the Schur product is formed with real_fj
@@ -348,15 +433,11 @@ __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
   for (int p = 0; p < len; ++p) {
     const int64_t r = r0 + p;
     TD Dp[25];
-#pragma unroll
-    for (int e = 0; e < 25; ++e) Dp[e] = lD[(r * 25 + e) * 32 + lane];
+    block_load<TD>(lD + r * DROW, int(lane), Dp);
     if (p > 0) {
       TB Lm[25], Um[25];
-#pragma unroll
-      for (int e = 0; e < 25; ++e) {
-        Lm[e] = lL[(r * 25 + e) * 32 + lane];
-        Um[e] = lU[((r - 1) * 25 + e) * 32 + lane];
-      }
+      block_load<TB>(lL + r * 25 * 32, int(lane), Lm);
+      block_load<TB>(lU + (r - 1) * 25 * 32, int(lane), Um);
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
         TD v[5];
@@ -375,24 +456,32 @@ __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
       }
     }
     if (!lu5_nopiv<TD>(Dp)) atomicOr(err, 2);
+    block_store<TD>(lD + r * DROW, int(lane), Dp);
 #pragma unroll
-    for (int e = 0; e < 25; ++e) {
-      lD[(r * 25 + e) * 32 + lane] = Dp[e];
-      prev[e] = Dp[e];
-    }
+    for (int k = 0; k < 5; ++k)
+      lD[r * DROW + (25 + k) * 32 + lane] = pivot_ok(Dp[6 * k]) ? TD(1) / Dp[6 * k] : TD(nanf(""));
+#pragma unroll
+    for (int e = 0; e < 25; ++e) prev[e] = Dp[e];
   }
 }
 
-// right-hand side of the rows of one colour: B - sum_outer F x_outer
+// right-hand side of the rows of one colour: B - sum_outer F x_outer; xt (may
+// be null) keeps the rows' own iterate for the relaxation, before the line
+// solve that follows overwrites it
 template <class TB, class TX>
 __global__ void k_lsgs_rhs(int64_t row_begin, int64_t nrows, LineView V,
                            const TB* __restrict__ lF, const TB* __restrict__ lB,
-                           const TX* __restrict__ x, TX* __restrict__ rhs,
+                           const TX* __restrict__ x, TX* __restrict__ rhs, TX* __restrict__ xt,
                            const LsgsCtl* __restrict__ ctl) {
   if (ctl->done) return;
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= nrows * 32) return;
   const int64_t r = row_begin + (i >> 5), lane = i & 31;
+  if (xt) {
+    const int64_t t = r * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) xt[5 * t + k] = x[5 * t + k];
+  }
   TX b[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) b[k] = TX(__ldcs(lB + (r * 5 + k) * 32 + lane));
@@ -439,209 +528,299 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait: false after ~2^24 polls (each poll may suspend the warp)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t it = 0; it < (1u << 24); ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-constexpr int LSGS_NST = 4;  // pipeline depth (rows in flight per group)
+constexpr int THOMAS_STAGES = 4;  // most stages in flight per group
+constexpr size_t THOMAS_SMEM_MAX = 227 * 1024;  // what a CTA may have
+constexpr int THOMAS_THREADS = 64;
 
+// a stage holds `rows` consecutive rows of a group
 template <class TB, class TD, class TX>
 struct ThomasStage {
-  static constexpr uint32_t d_bytes = 25 * 32 * sizeof(TD);
-  static constexpr uint32_t m_bytes = 25 * 32 * sizeof(TB);  // L (forward) or U (backward)
-  static constexpr uint32_t b_bytes = 5 * 32 * (sizeof(TX) > sizeof(TB) ? sizeof(TX) : sizeof(TB));
-  static constexpr uint32_t x_bytes = 5 * 32 * sizeof(TX);  // one row of the iterate
-  static constexpr uint32_t bytes = d_bytes + m_bytes + b_bytes + x_bytes;  // multiple of 16
+  static constexpr int rows = sizeof(TD) == 4 ? 4 : 2;
+  static constexpr uint32_t d_row = DROW * sizeof(TD);
+  static constexpr uint32_t m_row = 25 * 32 * sizeof(TB);  // L (forward) or U (backward)
+  static constexpr uint32_t b_row = 5 * 32 * (sizeof(TX) > sizeof(TB) ? sizeof(TX) : sizeof(TB));
+  static constexpr uint32_t m_off = rows * d_row, b_off = m_off + rows * m_row;
+  static constexpr uint32_t bytes = b_off + rows * b_row;  // multiple of 16
 };
+// shared memory: nst stages, their full and empty barriers, an abort flag
+// and the forward results of `rows` rows
 template <class TB, class TD, class TX>
-constexpr size_t thomas_smem_bytes() {
-  return size_t(LSGS_NST) * ThomasStage<TB, TD, TX>::bytes + 16 * LSGS_NST;
+constexpr size_t thomas_smem_bytes(int nst, int64_t rows) {
+  return size_t(nst) * ThomasStage<TB, TD, TX>::bytes + 16 * nst + 16 + size_t(rows) * 5 * 32 * sizeof(TX);
 }
 
 // block Thomas solve of the lines of groups [g0, g0+ng) (lineSolve,
-// linearSolverLSGS.loci:1523-1572), one warp per group of 32 lines, one
-// line per lane.  use_B: right-hand side B (start); save_xt: keep the
-// iterate before the solve for the relaxation.
+// linearSolverLSGS.loci:1523-1572), one CTA per group of 32 lines, one line
+// per lane of its first warp.  use_B: right-hand side B (start).
 //
-// A group's rows are contiguous ([row][entry][32 lanes]), so each row's
-// factored diagonal block, coupling block and right-hand side arrive as
-// bulk copies into shared memory, LSGS_NST rows ahead of the recurrence.
-// The iterate's row comes the same way: before the forward solve
-// overwrites it (kept for the relaxation) and, in the back substitution,
-// the forward result (written by this warp, then made visible to the copy
-// engine by a proxy fence).  Lane 0 issues the copies; every wait is
-// bounded and a wait that gives up sets bit 4 of err and ends the kernel
-// once the copies in flight landed.
-template <class TB, class TD, class TX>
-__global__ void __launch_bounds__(32)
-k_lsgs_thomas(int64_t g0, LineView V, const TD* __restrict__ lD, const TB* __restrict__ lL,
-              const TB* __restrict__ lU, const TX* __restrict__ rhs, const TB* __restrict__ lB,
-              int use_B, int save_xt, TX* __restrict__ x, TX* __restrict__ xt,
+// The 5x5 recurrence along a line is a serial chain: with 4,096 lines there
+// is less than one walking warp per SM and nothing hides what it waits for.
+// So the walking warp does the arithmetic alone: a second warp feeds it
+// (the rows of a group are contiguous, [row][block][32 lanes], and arrive as
+// bulk copies of a stage's rows, full/empty barriers), each row's blocks are
+// requested from shared memory before the row before is done, and the
+// forward results stay in shared memory (YS; lines too long for it keep them
+// in the spent right-hand-side rows).  Divisions are quotient()s; a chunk of
+// rows whose operands leave its range is done again with divisions.  An LSGS
+// iteration of 131,072 cells (64 rows, four solves with their right-hand
+// sides, MIXED) went from 397 to 174 us: a row's step from 0.66 to 0.21 us,
+// against about 0.1 us of its dependent FMAs.  Every wait is bounded; one that gives
+// up sets bit 4 of err and the abort flag, and the copies in flight land
+// before the CTA ends.
+template <class TB, class TD, class TX, bool YS>
+__global__ void __launch_bounds__(THOMAS_THREADS)
+k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* __restrict__ lD, const TB* __restrict__ lL,
+              const TB* __restrict__ lU, TX* rhs, const TB* __restrict__ lB, int use_B, TX* __restrict__ x,
               const LsgsCtl* __restrict__ ctl, int32_t* __restrict__ err) {
   using S = ThomasStage<TB, TD, TX>;
+  constexpr int R = S::rows;
+  static_assert(R % 2 == 0, "register sets alternate by row");
   if (ctl && ctl->done) return;
   extern __shared__ __align__(128) unsigned char th_smem[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(th_smem + size_t(LSGS_NST) * S::bytes);
-  auto stage = [&](int s) { return th_smem + size_t(s) * S::bytes; };
-  const int lane = threadIdx.x;
+  uint64_t* full = reinterpret_cast<uint64_t*>(th_smem + size_t(nst) * S::bytes);
+  uint64_t* empty = full + nst;
+  volatile int* dead = reinterpret_cast<volatile int*>(empty + nst);
+  TX* ysm = reinterpret_cast<TX*>(th_smem + size_t(nst) * S::bytes + 16 * nst + 16);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t g = g0 + blockIdx.x;
   const int len = V.lane_len[g * 32 + lane];
   const int glen = __reduce_max_sync(0xffffffffu, len);
+  const int nch = (glen + R - 1) / R;  // stages' worth of rows: chunk c holds rows R c ..
   const int64_t r0 = V.grp_row0[g];
-  if (lane == 0)
-    for (int s = 0; s < LSGS_NST; ++s) mbar_init(bar + s);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncwarp();
-  uint32_t phase = 0;  // bit s: parity of the next completion of stage s
-  int inflight = 0;    // bit s: stage s has copies outstanding
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < nst; ++s) mbar_init(full + s), mbar_init(empty + s);
+    *dead = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    for (uint32_t it = 0; it < (1u << 24); ++it) {
+      if (mbar_try_wait(bar, parity)) return true;
+      if (*dead) break;
+    }
+    return false;
+  };
+
+  if (warp == 1) {
+    // the chunks forward (D'_{p-1}, L_p and the right-hand side of each row
+    // p), then backward (D'_p and U_p)
+    if (lane == 0) {
+      int q = 0, s = 0;
+      uint32_t round = 0;  // uses of each stage before this one
+      for (; q < 2 * nch; ++q) {
+        if (round > 0 && !wait(empty + s, (round - 1) & 1)) break;
+        unsigned char* st = th_smem + size_t(s) * S::bytes;
+        const int c = q < nch ? q : 2 * nch - 1 - q;
+        const int64_t r = r0 + int64_t(R) * c;
+        const uint32_t n = uint32_t(min(R, glen - R * c));
+        if (q < nch) {
+          const uint32_t first = c == 0 ? 1 : 0;  // row 0 has no D' before it
+          const uint32_t bb = 5 * 32 * uint32_t(use_B ? sizeof(TB) : sizeof(TX));
+          mbar_expect_tx(full + s, (n - first) * S::d_row + n * (S::m_row + bb));
+          if (n > first) bulk_g2s(st + first * S::d_row, lD + (r - 1 + first) * DROW, (n - first) * S::d_row, full + s);
+          bulk_g2s(st + S::m_off, lL + r * 25 * 32, n * S::m_row, full + s);
+          bulk_g2s(st + S::b_off, use_B ? (const void*)(lB + r * 5 * 32) : (const void*)(rhs + r * 5 * 32), n * bb,
+                   full + s);
+        } else {
+          mbar_expect_tx(full + s, n * (S::d_row + S::m_row));
+          bulk_g2s(st, lD + r * DROW, n * S::d_row, full + s);
+          bulk_g2s(st + S::m_off, lU + r * 25 * 32, n * S::m_row, full + s);
+        }
+        if (++s == nst) s = 0, ++round;
+      }
+      if (q < 2 * nch) {
+        atomicOr(err, 4);
+        *dead = 1;
+      }
+      // the last use of every stage has landed before the CTA may end
+      for (int k = q > nst ? q - nst : 0; k < q; ++k)
+        for (uint32_t it = 0; it < (1u << 24) && !mbar_try_wait(full + k % nst, (k / nst) & 1); ++it) {
+        }
+    }
+    return;
+  }
+
+  static_assert(sizeof(TD) == sizeof(TX), "the factors and the iterate have one type");
+  // register sets: the next row's blocks beside this one's, except where both
+  // are FP64 (they would spill)
+  constexpr int NS = sizeof(TB) == 8 ? 1 : 2;
   bool ok = true;
-
-  // forward stage for row p: D'_{p-1}, L_p (p > 0) and the right-hand side
-  auto issue_fwd = [&](int p) {
-    const int s = p % LSGS_NST;
-    const int64_t r = r0 + p;
-    unsigned char* st = stage(s);
-    const uint32_t bb = 5 * 32 * uint32_t(use_B ? sizeof(TB) : sizeof(TX));
-    mbar_expect_tx(bar + s, (p > 0 ? S::d_bytes + S::m_bytes : 0) + bb + (save_xt ? S::x_bytes : 0));
-    if (save_xt) bulk_g2s(st + S::d_bytes + S::m_bytes + S::b_bytes, x + r * 32 * 5, S::x_bytes, bar + s);
-    if (p > 0) {
-      bulk_g2s(st, lD + (r - 1) * 25 * 32, S::d_bytes, bar + s);
-      bulk_g2s(st + S::d_bytes, lL + r * 25 * 32, S::m_bytes, bar + s);
-    }
-    if (use_B)
-      bulk_g2s(st + S::d_bytes + S::m_bytes, lB + r * 5 * 32, bb, bar + s);
-    else
-      bulk_g2s(st + S::d_bytes + S::m_bytes, rhs + r * 5 * 32, bb, bar + s);
-  };
-  // backward stage for row p: D'_p, U_p and the forward result y_p
-  auto issue_bwd = [&](int p) {
-    const int s = (glen - 1 - p) % LSGS_NST;
-    const int64_t r = r0 + p;
-    unsigned char* st = stage(s);
-    mbar_expect_tx(bar + s, S::d_bytes + S::m_bytes + S::x_bytes);
-    bulk_g2s(st, lD + r * 25 * 32, S::d_bytes, bar + s);
-    bulk_g2s(st + S::d_bytes, lU + r * 25 * 32, S::m_bytes, bar + s);
-    bulk_g2s(st + S::d_bytes + S::m_bytes + S::b_bytes, x + r * 32 * 5, S::x_bytes, bar + s);
-  };
-  auto wait_stage = [&](int s) {
-    const bool got = mbar_wait(bar + s, (phase >> s) & 1u);
-    if (got) {
-      phase ^= 1u << s;
-      inflight &= ~(1 << s);
-    }
-    return got;
-  };
-
-  // forward elimination: y_p = rhs_p - L_p D'_{p-1}^{-1} y_{p-1}
-  for (int p = 0; p < min(glen, LSGS_NST); ++p) {
-    if (lane == 0) issue_fwd(p);
-    inflight |= 1 << (p % LSGS_NST);
-  }
-  TX y[5];
-  for (int p = 0; p < glen && ok; ++p) {
-    const int s = p % LSGS_NST;
-    ok = __all_sync(0xffffffffu, wait_stage(s));
-    if (!ok) break;
-    const unsigned char* st = stage(s);
-    const TD* sD = reinterpret_cast<const TD*>(st) + lane;
-    const TB* sL = reinterpret_cast<const TB*>(st + S::d_bytes) + lane;
-    const int64_t t = (r0 + p) * 32 + lane;
-    TX yn[5];
-    if (use_B) {
-      const TB* sb = reinterpret_cast<const TB*>(st + S::d_bytes + S::m_bytes) + lane;
+  TD D[NS][25], RD[NS][5];  // factors and their pivots' reciprocals
+  TB M[NS][25];
+  TX B[NS][5];
+  int s = 0;  // the stage being read
+  uint32_t parity = 0;
+  uint32_t key = ~0u;  // of the chunk's dividends
+  // row j of the stage's chunk (row p of the group) into register set k
+  auto fetch = [&](int j, int p, int k, bool fwd) {
+    k %= NS;
+    const unsigned char* st = th_smem + size_t(s) * S::bytes;
+    const TD* sd = reinterpret_cast<const TD*>(st + j * S::d_row);
+    block_load<TD>(sd, lane, D[k]);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) yn[k] = TX(sb[k * 32]);
+    for (int e = 0; e < 5; ++e) RD[k][e] = sd[(25 + e) * 32 + lane];
+    block_load<TB>(reinterpret_cast<const TB*>(st + S::m_off + j * S::m_row), lane, M[k]);
+    if (!fwd) {
+#pragma unroll
+      for (int e = 0; e < 5; ++e) B[k][e] = YS ? ysm[(p * 5 + e) * 32 + lane] : rhs[((r0 + p) * 5 + e) * 32 + lane];
+    } else if (use_B) {
+      const TB* sb = reinterpret_cast<const TB*>(st + S::b_off) + j * 5 * 32 + lane;
+#pragma unroll
+      for (int e = 0; e < 5; ++e) B[k][e] = TX(sb[e * 32]);
     } else {
-      const TX* sb = reinterpret_cast<const TX*>(st + S::d_bytes + S::m_bytes) + lane;
+      const TX* sb = reinterpret_cast<const TX*>(st + S::b_off) + j * 5 * 32 + lane;
 #pragma unroll
-      for (int k = 0; k < 5; ++k) yn[k] = sb[k * 32];
+      for (int e = 0; e < 5; ++e) B[k][e] = sb[e * 32];
     }
-    if (p > 0 && p < len) {
-      TD Dm[25];
-#pragma unroll
-      for (int e = 0; e < 25; ++e) Dm[e] = sD[e * 32];
-      lu5_nopiv_solve<TD, TX>(Dm, y);
-#pragma unroll
-      for (int k = 0; k < 5; ++k)
-#pragma unroll
-        for (int j = 0; j < 5; ++j) yn[k] -= TX(sL[(5 * k + j) * 32]) * y[j];
-    }
-    TX xo[5];
-    if (save_xt) {
-      const TX* sx = reinterpret_cast<const TX*>(st + S::d_bytes + S::m_bytes + S::b_bytes) + 5 * lane;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) xo[k] = sx[k];
-    }
+  };
+  // on to the next chunk's stage; release: hands one back
+  auto advance = [&]() {
+    if (++s == nst) s = 0, parity ^= 1;
+    ok = wait(full + s, parity) && ok;
+  };
+  auto release = [&](int st) {
     __syncwarp();
-    if (lane == 0 && p + LSGS_NST < glen) issue_fwd(p + LSGS_NST);
-    if (p + LSGS_NST < glen) inflight |= 1 << s;
-    if (p < len) {
-      if (save_xt) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) xt[5 * t + k] = xo[k];
-      }
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        y[k] = yn[k];
-        x[5 * t + k] = yn[k];
-      }
+    if (lane == 0) mbar_arrive(empty + st);
+  };
+  // D'^{-1} v; a lane past its line's end computes on padding and keeps
+  // neither the result nor the key
+  auto solve = [&](int k, bool live, bool exact, TX* v) {
+    if (exact) {
+      lu5_nopiv_solve<TD, TX>(D[k], v);
+    } else {
+      uint32_t kk = ~0u;
+      lu5_recip_solve<TX>(D[k], RD[k], v, kk);
+      if (live) key = min(key, kk);
     }
-  }
-  // back substitution: x_p = D'_p^{-1} (y_p - U_p x_{p+1}); the forward
-  // results are read back through the copy engine
-  asm volatile("fence.proxy.async.global;" ::: "memory");
-  __syncwarp();
-  if (ok) {
-    for (int q = 0; q < min(glen, LSGS_NST); ++q) {
-      if (lane == 0) issue_bwd(glen - 1 - q);
-      inflight |= 1 << (q % LSGS_NST);
-    }
-    TX xn[5];
-    for (int q = 0; q < glen && ok; ++q) {
-      const int p = glen - 1 - q;
-      const int s = q % LSGS_NST;
-      ok = __all_sync(0xffffffffu, wait_stage(s));
-      if (!ok) break;
-      const unsigned char* st = stage(s);
-      const TD* sD = reinterpret_cast<const TD*>(st) + lane;
-      const TB* sU = reinterpret_cast<const TB*>(st + S::d_bytes) + lane;
-      const int64_t t = (r0 + p) * 32 + lane;
+  };
+  // forward elimination: y_p = rhs_p - L_p D'_{p-1}^{-1} y_{p-1}
+  TX y[5] = {TX(0), TX(0), TX(0), TX(0), TX(0)};
+  auto fwd_row = [&](int p, int k, bool first, bool exact) {
+    k %= NS;
+    const bool live = p < len;
+    TX yn[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) yn[e] = B[k][e];
+    if (!first) {
       TX v[5];
-      TD Dp[25];
-      if (p < len) {
-        const TX* sx = reinterpret_cast<const TX*>(st + S::d_bytes + S::m_bytes + S::b_bytes) + 5 * lane;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) v[k] = sx[k];
-        if (p < len - 1) {
+      for (int e = 0; e < 5; ++e) v[e] = y[e];
+      solve(k, live, exact, v);
 #pragma unroll
-          for (int k = 0; k < 5; ++k)
+      for (int e = 0; e < 5; ++e)
 #pragma unroll
-            for (int j = 0; j < 5; ++j) v[k] -= TX(sU[(5 * k + j) * 32]) * xn[j];
-        }
-#pragma unroll
-        for (int e = 0; e < 25; ++e) Dp[e] = sD[e * 32];
-      }
-      __syncwarp();
-      if (lane == 0 && q + LSGS_NST < glen) issue_bwd(p - LSGS_NST);
-      if (q + LSGS_NST < glen) inflight |= 1 << s;
-      if (p < len) {
-        lu5_nopiv_solve<TD, TX>(Dp, v);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          x[5 * t + k] = v[k];
-          xn[k] = v[k];
-        }
-      }
+        for (int j = 0; j < 5; ++j) yn[e] -= TX(M[k][5 * e + j]) * v[j];
     }
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+      y[e] = live ? yn[e] : y[e];
+      if (YS)
+        ysm[(p * 5 + e) * 32 + lane] = yn[e];
+      else
+        rhs[((r0 + p) * 5 + e) * 32 + lane] = yn[e];
+    }
+  };
+  // back substitution: x_p = D'_p^{-1} (y_p - U_p x_{p+1}); a line's last
+  // row has U = 0 and comes before any x of its line (xn = 0)
+  TX xn[5] = {TX(0), TX(0), TX(0), TX(0), TX(0)};
+  auto bwd_row = [&](int p, int k, bool exact) {
+    k %= NS;
+    const bool live = p < len;
+    TX v[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) v[e] = B[k][e];
+#pragma unroll
+    for (int e = 0; e < 5; ++e)
+#pragma unroll
+      for (int j = 0; j < 5; ++j) v[e] -= TX(M[k][5 * e + j]) * xn[j];
+    solve(k, live, exact, v);
+    TX* xo = x + 5 * ((r0 + p) * 32 + lane);
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+      xn[e] = live ? v[e] : xn[e];
+      if (live) xo[e] = v[e];
+    }
+  };
+  // whether a chunk has to be done again with divisions: a dividend too
+  // small, a pivot out of range or an overflow (v: the chunk's last row)
+  auto inexact = [&](const TX* v) {
+    const TX sum = ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+    const bool again = tiny<TX>(key) || sum != sum;
+    key = ~0u;
+    return __any_sync(0xffffffffu, again);
+  };
+  // n rows of chunk c, forward or backward; next: another chunk follows in
+  // the same direction, whose stage is waited for before this chunk's last
+  // row.  On entry the first row's blocks are in registers (NS == 2).
+  auto chunk = [&](int c, auto full_chunk, auto forward, bool next) {
+    constexpr bool FULL = decltype(full_chunk)::value, FWD = decltype(forward)::value;
+    const int n = FULL ? R : glen - R * c;
+    TX v0[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) v0[e] = FWD ? y[e] : xn[e];
+    const int sc = s;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int j = FWD ? i : R - 1 - i, p = R * c + j;
+      if (!FULL && j >= n) continue;
+      if (NS == 1) fetch(j, p, 0, FWD);
+      if (i + 1 < R && (FULL || !FWD || j + 1 < n)) {
+        if (NS == 2) fetch(FWD ? j + 1 : j - 1, FWD ? p + 1 : p - 1, (j + 1) & 1, FWD);
+      } else if (next) {
+        advance();
+        if (NS == 2) fetch(FWD ? 0 : R - 1, FWD ? p + 1 : p - 1, (j + 1) & 1, FWD);
+      }
+      if (FWD)
+        fwd_row(p, j & 1, j == 0 && c == 0, false);
+      else
+        bwd_row(p, j & 1, false);
+    }
+    if (inexact(FWD ? y : xn)) {
+      const int sn = s;
+      s = sc;
+#pragma unroll
+      for (int e = 0; e < 5; ++e) (FWD ? y : xn)[e] = v0[e];
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const int j = FWD ? i : n - 1 - i, p = R * c + j;
+        fetch(j, p, 0, FWD);
+        if (FWD)
+          fwd_row(p, 0, p == 0, true);
+        else
+          bwd_row(p, 0, true);
+      }
+      s = sn;
+      key = ~0u;
+      // the next row's blocks again, overwritten by the second pass
+      if (NS == 2 && next) fetch(FWD ? 0 : R - 1, FWD ? R * c + R : R * c - 1, FWD ? 0 : 1, FWD);
+    }
+    release(sc);
+  };
+  using yes = std::true_type;
+  using no = std::false_type;
+  if (nch > 0) {
+    const int nfull = glen / R;
+    ok = wait(full, 0);
+    if (NS == 2) fetch(0, 0, 0, true);
+    for (int c = 0; c < nfull && ok; ++c) chunk(c, yes{}, yes{}, c + 1 < nch);
+    if (nfull < nch && ok) chunk(nfull, no{}, yes{}, false);
+    if (ok) advance();
+    if (NS == 2 && ok) {
+      if ((glen - 1) & 1)
+        fetch((glen - 1) % R, glen - 1, 1, false);
+      else
+        fetch((glen - 1) % R, glen - 1, 0, false);
+    }
+    if (nfull < nch && ok) chunk(nfull, no{}, no{}, nfull > 0);
+    for (int c = nfull - 1; c >= 0 && ok; --c) chunk(c, yes{}, no{}, c > 0);
   }
   if (!ok) {
-    if (lane == 0) atomicOr(err, 4);
-    // let the copies in flight land before the block's shared memory goes
-    for (int s = 0; s < LSGS_NST; ++s)
-      if (inflight & (1 << s)) mbar_wait(bar + s, (phase >> s) & 1u);
+    atomicOr(err, 4);
+    *dead = 1;
   }
 }
 
@@ -758,6 +937,37 @@ int lsgs_assemble(fpsi_ctx* x) {
   }
 }
 
+// The line solves of ng groups from g0.  Stages per group: what half an SM's
+// shared memory holds beside the longest line's forward results (two CTAs
+// per SM), or the whole of it where the groups do not fill the SMs twice
+// anyway or half holds fewer than two; lines too long for that keep their
+// forward results in memory.
+template <class TB, class TD, class TX>
+static int launch_thomas(fpsi_ctx* x, int64_t g0, int64_t ng, bool use_B, const dev::LsgsCtl* ctl) {
+  auto stages = [&](size_t smem, int64_t ylen) {
+    int n = 0;
+    while (n < dev::THOMAS_STAGES && dev::thomas_smem_bytes<TB, TD, TX>(n + 1, ylen) <= smem) ++n;
+    return n;
+  };
+  const size_t half = dev::THOMAS_SMEM_MAX / 2 - 1024, whole = dev::THOMAS_SMEM_MAX;
+  int64_t ylen = x->LY.max_len;
+  int nst = stages(half, ylen);
+  if (nst < 2 || ng <= x->nsm) nst = stages(whole, ylen);
+  if (nst < 2) {
+    ylen = 0;
+    nst = stages(half, ylen);
+  }
+  auto k = ylen > 0 ? dev::k_lsgs_thomas<TB, TD, TX, true> : dev::k_lsgs_thomas<TB, TD, TX, false>;
+  const size_t smem = dev::thomas_smem_bytes<TB, TD, TX>(nst, ylen);
+  FPSI_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  prof_begin(x, "lsgs_thomas");
+  k<<<unsigned(ng), dev::THOMAS_THREADS, smem, x->stream>>>(
+      nst, g0, line_view(x), (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, (TX*)x->d_lrhs,
+      (const TB*)x->d_lB, use_B, (TX*)x->d_lx, ctl, x->d_err);
+  prof_end(x);
+  return FPSI_OK;
+}
+
 template <class TB, class TD, class TX>
 static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
   const LineLayout& Y = x->LY;
@@ -768,17 +978,8 @@ static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
   TX* X = (TX*)x->d_lx;
   TX* XT = (TX*)x->d_lxt;
   dev::k_lsgs_init<<<1, 1, 0, s>>>(ctl, x->P.lsgs_relaxation);
-  constexpr size_t th_smem = dev::thomas_smem_bytes<TB, TD, TX>();
-  if (th_smem > 48 * 1024)
-    FPSI_CUDA_TRY(cudaFuncSetAttribute(dev::k_lsgs_thomas<TB, TD, TX>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(th_smem)));
-  if (jacobi_start) {
-    prof_begin(x, "lsgs_thomas");
-    dev::k_lsgs_thomas<TB, TD, TX><<<unsigned(Y.ngroups), 32, th_smem, s>>>(
-        0, V, (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, nullptr,
-        (const TB*)x->d_lB, 1, 0, X, XT, nullptr, x->d_err);
-    prof_end(x);
-  }
+  int rc;
+  if (jacobi_start && (rc = launch_thomas<TB, TD, TX>(x, 0, Y.ngroups, true, nullptr))) return rc;
   const int K = Y.ncolours;
   const int nblk = int(nblocks(nt, dev::RELAX_THREADS));
   for (int it = 0; it < x->P.lsgs_max_iter; ++it) {
@@ -791,13 +992,10 @@ static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
         const int64_t re = Y.grp_row0[g0 + ng - 1] + Y.grp_len[g0 + ng - 1];
         prof_begin(x, "lsgs_rhs");
         dev::k_lsgs_rhs<TB, TX><<<nblocks((re - rb) * 32, 128), 128, 0, s>>>(
-            rb, re - rb, V, (const TB*)x->d_lF, (const TB*)x->d_lB, X, (TX*)x->d_lrhs, ctl);
+            rb, re - rb, V, (const TB*)x->d_lF, (const TB*)x->d_lB, X, (TX*)x->d_lrhs,
+            pass == 1 ? XT : nullptr, ctl);
         prof_end(x);
-        prof_begin(x, "lsgs_thomas");
-        dev::k_lsgs_thomas<TB, TD, TX><<<unsigned(ng), 32, th_smem, s>>>(
-            g0, V, (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU,
-            (const TX*)x->d_lrhs, (const TB*)x->d_lB, 0, pass == 1 ? 1 : 0, X, XT, ctl, x->d_err);
-        prof_end(x);
+        if ((rc = launch_thomas<TB, TD, TX>(x, g0, ng, false, ctl))) return rc;
       }
     prof_begin(x, "lsgs_relax");
     dev::k_lsgs_relax<TX><<<nblk, dev::RELAX_THREADS, 0, s>>>(nt, X, XT, ctl, x->d_lpart);
