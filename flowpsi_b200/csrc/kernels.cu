@@ -1444,37 +1444,56 @@ struct SweepView {
 // so every slot store fills whole 32 B sectors.
 //
 // Face blocks reach the threads through shared memory: for face entry e of
-// its 32 cells, a warp copies the (fjp, fjm) pairs with consecutive lanes on
-// consecutive words of each 25-entry block, then every thread adds its own
-// pair.  Each cell still sums its faces in list order.
+// its 32 cells, a warp copies the face records with consecutive lanes on
+// consecutive words, then every thread adds its own.  Compact records come
+// as 16 B asynchronous copies into two buffers, entry e + 1 in flight while
+// entry e is expanded (no registers hold it); explicit (fjp, fjm) pairs
+// through registers.  Each cell still sums its faces in list order.  Bound by
+// the latency of the gathered records: 663,552 tets MIXED with the diagonal
+// blocks kept take 0.154 ms (0.202 with the records through registers and
+// the blocks' rows stored lane by lane), 1.57 M 0.347 (0.450), 592,704 hexes
+// 0.149 (0.182), 663,552 tets FP64 0.234 (0.335).  Four CTAs per SM (three
+// FP64) rather than five, whose 96 registers cost 0.163, or six (spills, 0.208).
 constexpr int ASM_THREADS = 128;
 constexpr int ASM_STRIDE = 33;  // shared row stride: 32 cells + 1 (no bank conflicts)
 constexpr int ASM_BATCH = 10;   // loads in flight per lane while staging
+// compact records move in 16 B units, stored record-major with an odd stride
+// of asm_rs16 units so that a quarter warp's 16 B accesses hit distinct banks
 template <class TB>
+constexpr int asm_u16() { return int(CK_FACE * sizeof(TB) / 16); }
+template <class TB>
+constexpr int asm_rs16() { return asm_u16<TB>() + 1; }
+// bytes of one warp's staging area; it also stages the diagonal blocks' rows
+template <class TB, bool CPT>
+constexpr size_t asm_warp_bytes() {
+  return CPT ? size_t(2) * 32 * asm_rs16<TB>() * 16 : size_t(50) * ASM_STRIDE * sizeof(TB);
+}
+template <class TB, bool CPT>
 constexpr size_t asm_smem_bytes() {
-  return size_t(ASM_THREADS / 32) * 50 * ASM_STRIDE * sizeof(TB);
+  return size_t(ASM_THREADS / 32) * asm_warp_bytes<TB, CPT>();
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src)
+               : "memory");
 }
 
 // CPT: the face blocks come as compact records (fjc, CK_FACE values per
 // face) and the slots are written compact (CK_SLOT values); otherwise as
 // explicit (fjp, fjm) pairs into 25-value slots.
 template <class TB, class TX, bool CPT>
-__global__ void __launch_bounds__(ASM_THREADS, sizeof(TB) == 4 ? (CPT ? 5 : 6) : 4)
+__global__ void __launch_bounds__(ASM_THREADS, sizeof(TB) == 4 ? (CPT ? 4 : 6) : (CPT ? 3 : 4))
 k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* __restrict__ src,
            const double* __restrict__ dtau, const TB* __restrict__ fjp, const TB* __restrict__ fjm,
            const TB* __restrict__ fjc, Gas g, TB* __restrict__ luc, TB* __restrict__ bcv,
            int32_t* __restrict__ pvv, TB* __restrict__ aoff, TB* __restrict__ Dout, TX* __restrict__ x,
            int32_t* __restrict__ err, double dcoef, const TB* __restrict__ bjac) {
   constexpr int RW = 50;  // words staged per face (explicit blocks)
-  // compact records move in 16 B units: U16 per record, stored record-major
-  // with an odd stride of RS16 units so that a quarter warp's 16 B accesses
-  // hit distinct banks
-  constexpr int U16 = int(CK_FACE * sizeof(TB) / 16), RS16 = U16 + 1;
+  constexpr int U16 = asm_u16<TB>(), RS16 = asm_rs16<TB>();
   static_assert(CK_FACE * sizeof(TB) % 16 == 0, "a compact record is whole 16 B units");
-  static_assert(32 * RS16 * 16 <= 50 * ASM_STRIDE * sizeof(TB), "fits the warp's staging area");
+  static_assert(32 * 25 * sizeof(TB) <= asm_warp_bytes<TB, CPT>(), "the diagonal blocks fit the staging area");
   extern __shared__ __align__(16) unsigned char asm_smem[];
-  TB* st = reinterpret_cast<TB*>(asm_smem) + (threadIdx.x >> 5) * (50 * ASM_STRIDE);
-  uint4* st4 = reinterpret_cast<uint4*>(asm_smem + (threadIdx.x >> 5) * size_t(32 * RS16 * 16));
+  TB* st = reinterpret_cast<TB*>(asm_smem + (threadIdx.x >> 5) * asm_warp_bytes<TB, CPT>());
+  uint4* st4 = reinterpret_cast<uint4*>(st);
   const int lane = threadIdx.x & 31;
   const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool active = c < M.nc;
@@ -1494,31 +1513,34 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
 #pragma unroll
   for (int k = 0; k < 25; ++k) sJ[k] = TB(0);
   int64_t slot = 0;
+  // the warp's 32 records of one entry as 32 * U16 units of 16 B, U16 per
+  // lane, into buffer b (lanes without an entry read face 0; their units are
+  // never used)
+  auto issue = [&](int32_t entry, int b) {
+#pragma unroll
+    for (int u = 0; u < U16; ++u) {
+      const int idx = lane + 32 * u;
+      const int L = idx / U16, j = idx - U16 * L;
+      const int32_t ent = __shfl_sync(0xffffffffu, entry, L);
+      const int64_t f = ent >= 0 ? int64_t(ent >> 1) : 0;
+      cp_async16(st4 + (b * 32 + L) * RS16 + j, reinterpret_cast<const uint4*>(fjc + CK_FACE * f) + j);
+    }
+  };
+  auto entry = [&](int e) { return active && e < maxdeg ? __ldg(M.ecf + int64_t(e) * M.nc + c) : -1; };
+  int32_t ent_next = -1, ent_after = -1;
+  if constexpr (CPT) {
+    ent_next = entry(0);
+    ent_after = entry(1);
+    if (maxdeg > 0) issue(ent_next, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   for (int e = 0; e < maxdeg; ++e) {
-    const int32_t my_ent = e < deg ? M.cf[e0 + e] : -1;
+    const int32_t my_ent = CPT ? ent_next : e < deg ? M.cf[e0 + e] : -1;
     if constexpr (CPT) {
-      // the warp's 32 records as 32 * U16 units of 16 B, U16 per lane, all
-      // in flight together (lanes without an entry read face 0; their units
-      // are never used)
-      constexpr int HALF = U16 > 6 ? U16 / 2 : U16;  // units held in registers at once
-#pragma unroll
-      for (int h = 0; h < U16; h += HALF) {
-        uint4 v[HALF];
-#pragma unroll
-        for (int u = 0; u < HALF; ++u) {
-          const int idx = lane + 32 * (h + u);
-          const int L = idx / U16, j = idx - U16 * L;
-          const int32_t ent = __shfl_sync(0xffffffffu, my_ent, L);
-          const int64_t f = ent >= 0 ? int64_t(ent >> 1) : 0;
-          v[u] = __ldg(reinterpret_cast<const uint4*>(fjc + CK_FACE * f) + j);
-        }
-#pragma unroll
-        for (int u = 0; u < HALF; ++u) {
-          const int idx = lane + 32 * (h + u);
-          const int L = idx / U16, j = idx - U16 * L;
-          st4[L * RS16 + j] = v[u];
-        }
-      }
+      ent_next = ent_after;
+      ent_after = entry(e + 2);
+      if (e + 1 < maxdeg) issue(ent_next, (e + 1) & 1);
+      asm volatile("cp.async.commit_group;\n cp.async.wait_group 1;" ::: "memory");
     } else {
       // 32 RW words per round, RW per lane, in batches of ASM_BATCH
       // independent loads (fjm is allocated for every face, so every address
@@ -1550,7 +1572,7 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
       const int64_t f = my_ent >> 1;
       TB r[CK_FACE];
 #pragma unroll
-      for (int j = 0; j < U16; ++j) reinterpret_cast<uint4*>(r)[j] = st4[lane * RS16 + j];
+      for (int j = 0; j < U16; ++j) reinterpret_cast<uint4*>(r)[j] = st4[((e & 1) * 32 + lane) * RS16 + j];
       TB* ao = aoff ? aoff + CK_SLOT * ck.ebp + slot * CK_SLOT * ld + i : nullptr;
       TB Mb[25];
       if (my_ent & 1) {
@@ -1606,8 +1628,7 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
     }
     __syncwarp();
   }
-  if (!active) return;
-  if (bjac) {  // difference blocks of the total-pressure and fixed-mass inflows
+  if (active && bjac) {  // difference blocks of the total-pressure and fixed-mass inflows
     for (int e = 0; e < deg; ++e) {
       const int64_t f = M.cf[e0 + e] >> 1;
       if (f < M.nfi || !fd_jacobian_kind(M.bcs[-M.cr[f] - 1].kind)) continue;
@@ -1619,9 +1640,10 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
   TB D[25];
 #pragma unroll
   for (int i = 0; i < 25; ++i) D[i] = -sJ[i];
-  const Q5 qc = load_q(q, c);
+  const int64_t ca = active ? c : M.nc - 1;  // idle lanes follow with another cell's values
+  const Q5 qc = load_q(q, ca);
   // V / dtau (steady, solverLinearSystem.loci:176-215), 1.5 V / dtau (BDF2, :376-435)
-  const double coef = dcoef * M.vol[c] / dtau[c];
+  const double coef = dcoef * M.vol[ca] / dtau[ca];
   const double T = qc.T, rP = 1.0 / (g.Rt * T);
   const double rho = (qc.p + g.pamb) * rP;
   const double rT = -rho / T;
@@ -1644,10 +1666,19 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
     D[21 + r] = TB(double(D[21 + r]) + coef * rho * U[r]);
   }
   if (Dout) {
-    TB* o = Dout + 25 * c;
+    // the warp's 32 blocks are one contiguous range of memory: through the
+    // staging area (row stride 25 words: no bank conflicts), consecutive lanes
+    // on consecutive words
 #pragma unroll
-    for (int i = 0; i < 25; ++i) o[i] = D[i];
+    for (int k = 0; k < 25; ++k) st[25 * lane + k] = D[k];
+    __syncwarp();
+    const int64_t w0 = 25 * (c - lane);
+    const int nw = int(min(int64_t(32 * 25), 25 * M.nc - w0));
+#pragma unroll
+    for (int k = 0; k < 25; ++k)
+      if (lane + 32 * k < nw) Dout[w0 + lane + 32 * k] = st[lane + 32 * k];
   }
+  if (!active) return;
   int piv[5];
   if (!lu5<TB>(D, piv)) atomicOr(err, 1);
   int pv = 0;
@@ -2274,7 +2305,7 @@ static bool compact_blocks(const fpsi_ctx* x) {
 
 template <class TB, class TX, bool CPT>
 static void launch_assemble_kernel(fpsi_ctx* x, const dev::MeshView& M, const dev::Gas& g) {
-  constexpr size_t smem = dev::asm_smem_bytes<TB>();
+  constexpr size_t smem = dev::asm_smem_bytes<TB, CPT>();
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(dev::k_assemble<TB, TX, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(smem));
