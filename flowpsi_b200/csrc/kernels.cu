@@ -23,6 +23,7 @@
 
 #include "fpsi_internal.h"
 #include "kernels.cuh"
+#include "pdl.cuh"
 #include "physics.cuh"
 
 namespace fpsi {
@@ -1722,17 +1723,6 @@ __global__ void k_jacobi_start(ColInfo ck, const TB* __restrict__ luc,
   for (int k = 0; k < 5; ++k) x[5 * (ck.cb + i) + k] = y[k];
 }
 
-// ---------------------------------------------------------------------------
-// programmatic dependent launch: a grid launched with launch_after may start
-// while the grid before it drains; what it touches before pdl_wait must not
-// be written by any grid that can still be running.  Both are no-ops in a
-// plain launch.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 constexpr int SGS_THREADS = 128;
 
 // ---------------------------------------------------------------------------
@@ -2405,18 +2395,8 @@ static cudaError_t launch_sgs_pass(fpsi_ctx* x, const ColInfo& ck, bool after) {
     if (grid > int64_t(dev::sgs_ctas<TB, TX, CPT, MS>()) * x->nsm)
       return launch_sgs_pass<TB, TX, CPT, 0>(x, ck, after);
   }
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(grid));
-  cfg.blockDim = dim3(dev::SGS_THREADS);
-  cfg.stream = x->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = after ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, dev::k_sgs_colour<TB, TX, CPT, MS>, ck, (const int32_t*)x->d_nbr,
-                            (const TB*)x->d_aoff, (const TB*)x->d_luc, (const TB*)x->d_bc,
-                            (const int32_t*)x->d_pv, (TX*)x->d_x);
+  return launch_grid(x, after, dev::k_sgs_colour<TB, TX, CPT, MS>, grid, dev::SGS_THREADS, 0, ck, x->d_nbr,
+                     (const TB*)x->d_aoff, (const TB*)x->d_luc, (const TB*)x->d_bc, x->d_pv, (TX*)x->d_x);
 }
 
 template <class TB, class TX>
@@ -2434,7 +2414,7 @@ static int launch_sgs_t(fpsi_ctx* x, int sweeps) {
         const int k = pass == 0 ? kk : K - 1 - kk;
         const ColInfo ck = col_info(x, k);
         if (ck.n == 0 || k == last) continue;
-        const bool after = last >= 0 && !x->profiling;
+        const bool after = last >= 0;
         last = k;
         prof_begin(x, "sgs_colour");
         cudaError_t e;

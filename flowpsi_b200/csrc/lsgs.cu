@@ -24,6 +24,7 @@
 
 #include "fpsi_internal.h"
 #include "kernels.cuh"
+#include "pdl.cuh"
 
 namespace fpsi {
 
@@ -333,21 +334,23 @@ __device__ __forceinline__ bool tiny(uint32_t k) {
 template <class TB, class TD>
 __global__ void k_lsgs_scatter(int64_t nt, const int32_t* __restrict__ c_of_t,
                                const int32_t* __restrict__ cf_off, const int32_t* __restrict__ cf,
-                               LineView V, const TB* __restrict__ D, const TB* __restrict__ fjp,
-                               const TB* __restrict__ fjm, const double* __restrict__ src,
+                               LineView V, const TB* D, const TB* fjp,
+                               const TB* fjm, const double* src,
                                TD* __restrict__ lD, TB* __restrict__ lL, TB* __restrict__ lU,
                                TB* __restrict__ lF, TB* __restrict__ lB) {
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (t >= nt) return;
   const int64_t c = c_of_t[t];
   if (c < 0) return;
   const int64_t r = t >> 5, lane = t & 31;
   TD d[25];
 #pragma unroll
-  for (int e = 0; e < 25; ++e) d[e] = TD(__ldg(D + 25 * c + e));
+  for (int e = 0; e < 25; ++e) d[e] = TD(D[25 * c + e]);
   block_store<TD>(lD + r * DROW, int(lane), d);
 #pragma unroll
-  for (int k = 0; k < 5; ++k) lB[(r * 5 + k) * 32 + lane] = TB(__ldg(src + 5 * c + k));
+  for (int k = 0; k < 5; ++k) lB[(r * 5 + k) * 32 + lane] = TB(src[5 * c + k]);
   for (int32_t e = cf_off[c]; e < cf_off[c + 1]; ++e) {
     const int ro = V.role[e];
     if (ro == 0) continue;
@@ -357,7 +360,7 @@ __global__ void k_lsgs_scatter(int64_t nt, const int32_t* __restrict__ c_of_t,
     const TB* A = neg ? fjp + 25 * f : fjm + 25 * f;
     TB b[25];
 #pragma unroll
-    for (int k = 0; k < 25; ++k) b[k] = neg ? TB(-__ldg(A + k)) : __ldg(A + k);
+    for (int k = 0; k < 25; ++k) b[k] = neg ? TB(-A[k]) : A[k];
     if (ro < 3) {
       block_store<TB>((ro == 1 ? lL : lU) + r * 25 * 32, int(lane), b);
     } else {
@@ -422,9 +425,11 @@ __device__ __forceinline__ void lu5_recip_solve(const T* A, const T* r, T* y, ui
 // (TB) intermediates.
 template <class TB, class TD>
 __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
-                            const TB* __restrict__ lL, const TB* __restrict__ lU,
+                            const TB* lL, const TB* lU,
                             int32_t* __restrict__ err) {
   const int64_t gl = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (gl >= ngroups * 32) return;
   const int64_t g = gl >> 5, lane = gl & 31;
   const int len = V.lane_len[gl];
@@ -468,34 +473,46 @@ __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
 // right-hand side of the rows of one colour: B - sum_outer F x_outer; xt (may
 // be null) keeps the rows' own iterate for the relaxation, before the line
 // solve that follows overwrites it
+// The system is complete before a solve's first launch, so B, the neighbour
+// ids and the first coupling are read before the wait for the line solve
+// whose iterate the rows take.
 template <class TB, class TX>
-__global__ void k_lsgs_rhs(int64_t row_begin, int64_t nrows, LineView V,
-                           const TB* __restrict__ lF, const TB* __restrict__ lB,
-                           const TX* __restrict__ x, TX* __restrict__ rhs, TX* __restrict__ xt,
-                           const LsgsCtl* __restrict__ ctl) {
-  if (ctl->done) return;
+__global__ void k_lsgs_rhs(int64_t row_begin, int64_t nrows, LineView V, const TB* lF, const TB* lB, const TX* x,
+                           TX* rhs, TX* xt, const LsgsCtl* ctl) {
+  pdl_trigger();
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= nrows * 32) return;
   const int64_t r = row_begin + (i >> 5), lane = i & 31;
+  const int32_t* on = V.onbr + r * V.mout * 32 + lane;
+  const TB* F = lF + r * V.mout * 25 * 32 + lane;
+  TX b[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) b[k] = TX(__ldcs(lB + (r * 5 + k) * 32 + lane));
+  int32_t o = on[0];
+  TB f[25];
+#pragma unroll
+  for (int k = 0; k < 25; ++k) f[k] = __ldcs(F + k * 32);
+  pdl_wait();
+  if (ctl->done) return;
   if (xt) {
     const int64_t t = r * 32 + lane;
 #pragma unroll
     for (int k = 0; k < 5; ++k) xt[5 * t + k] = x[5 * t + k];
   }
-  TX b[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) b[k] = TX(__ldcs(lB + (r * 5 + k) * 32 + lane));
-  for (int s = 0; s < V.mout; ++s) {
-    const int32_t o = V.onbr[(r * V.mout + s) * 32 + lane];
-    if (o < 0) break;
+  for (int s = 0; s < V.mout && o >= 0; ++s) {
+    const int32_t onext = s + 1 < V.mout ? on[(s + 1) * 32] : -1;
     TX xo[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) xo[k] = x[5 * int64_t(o) + k];
-    const TB* F = lF + (r * V.mout + s) * 25 * 32 + lane;
+    if (s > 0) {
+#pragma unroll
+      for (int k = 0; k < 25; ++k) f[k] = __ldcs(F + (s * 25 + k) * 32);
+    }
 #pragma unroll
     for (int k = 0; k < 5; ++k)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) b[k] -= TX(__ldcs(F + (5 * k + j) * 32)) * xo[j];
+      for (int j = 0; j < 5; ++j) b[k] -= TX(f[5 * k + j]) * xo[j];
+    o = onext;
   }
 #pragma unroll
   for (int k = 0; k < 5; ++k) rhs[(r * 5 + k) * 32 + lane] = b[k];
@@ -573,12 +590,14 @@ constexpr size_t thomas_smem_bytes(int nst, int64_t rows) {
 // before the CTA ends.
 template <class TB, class TD, class TX, bool YS>
 __global__ void __launch_bounds__(THOMAS_THREADS)
-k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* __restrict__ lD, const TB* __restrict__ lL,
-              const TB* __restrict__ lU, TX* rhs, const TB* __restrict__ lB, int use_B, TX* __restrict__ x,
-              const LsgsCtl* __restrict__ ctl, int32_t* __restrict__ err) {
+k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* lD, const TB* lL,
+              const TB* lU, TX* rhs, const TB* lB, int use_B, TX* x,
+              const LsgsCtl* ctl, int32_t* __restrict__ err) {
   using S = ThomasStage<TB, TD, TX>;
   constexpr int R = S::rows;
   static_assert(R % 2 == 0, "register sets alternate by row");
+  pdl_trigger();
+  pdl_wait();
   if (ctl && ctl->done) return;
   extern __shared__ __align__(128) unsigned char th_smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(th_smem + size_t(nst) * S::bytes);
@@ -829,8 +848,10 @@ constexpr int RELAX_THREADS = 256;
 // X = w X + (1-w) X_t and the block partial of ||X - X_t||^2 (:1868-1874)
 template <class TX>
 __global__ void __launch_bounds__(RELAX_THREADS)
-k_lsgs_relax(int64_t nt, TX* __restrict__ x, const TX* __restrict__ xt,
-             const LsgsCtl* __restrict__ ctl, double* __restrict__ part) {
+k_lsgs_relax(int64_t nt, TX* x, const TX* xt,
+             const LsgsCtl* ctl, double* part) {
+  pdl_trigger();
+  pdl_wait();
   if (ctl->done) return;
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const double w = ctl->w;
@@ -856,8 +877,10 @@ k_lsgs_relax(int64_t nt, TX* __restrict__ x, const TX* __restrict__ xt,
 }
 
 // residual, adaptive relaxation and stopping test (:1923-1947)
-__global__ void k_lsgs_control(const double* __restrict__ part, int nblk, double abs_tol,
-                               double rel_tol, LsgsCtl* __restrict__ ctl) {
+__global__ void k_lsgs_control(const double* part, int nblk, double abs_tol,
+                               double rel_tol, LsgsCtl* ctl) {
+  pdl_trigger();
+  pdl_wait();
   if (ctl->done) return;
   __shared__ double sh[RELAX_THREADS];
   double s = 0;
@@ -910,16 +933,15 @@ dev::LineView line_view(const fpsi_ctx* x) {
 template <class TB, class TD, class TX>
 static int lsgs_assemble_t(fpsi_ctx* x) {
   const LineLayout& Y = x->LY;
-  cudaStream_t s = x->stream;
   const dev::LineView V = line_view(x);
   prof_begin(x, "lsgs_scatter");
-  dev::k_lsgs_scatter<TB, TD><<<nblocks(Y.nrows * 32, 128), 128, 0, s>>>(
+  launch_chain(x, dev::k_lsgs_scatter<TB, TD>, nblocks(Y.nrows * 32, 128), 128, 0,
       Y.nrows * 32, x->d_lct, x->d_cf_off, x->d_cf, V, (const TB*)x->d_D, (const TB*)x->d_fjp,
       (const TB*)x->d_fjm, x->d_src, (TD*)x->d_lD, (TB*)x->d_lL, (TB*)x->d_lU, (TB*)x->d_lF,
       (TB*)x->d_lB);
   prof_end(x);
   prof_begin(x, "lsgs_prep");
-  dev::k_lsgs_prep<TB, TD><<<nblocks(Y.ngroups * 32, 64), 64, 0, s>>>(
+  launch_chain(x, dev::k_lsgs_prep<TB, TD>, nblocks(Y.ngroups * 32, 64), 64, 0,
       Y.ngroups, V, (TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, x->d_err);
   prof_end(x);
   FPSI_CUDA_TRY(cudaGetLastError());
@@ -961,8 +983,7 @@ static int launch_thomas(fpsi_ctx* x, int64_t g0, int64_t ng, bool use_B, const 
   const size_t smem = dev::thomas_smem_bytes<TB, TD, TX>(nst, ylen);
   FPSI_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   prof_begin(x, "lsgs_thomas");
-  k<<<unsigned(ng), dev::THOMAS_THREADS, smem, x->stream>>>(
-      nst, g0, line_view(x), (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, (TX*)x->d_lrhs,
+  launch_chain(x, k, ng, dev::THOMAS_THREADS, smem, nst, g0, line_view(x), (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, (TX*)x->d_lrhs,
       (const TB*)x->d_lB, use_B, (TX*)x->d_lx, ctl, x->d_err);
   prof_end(x);
   return FPSI_OK;
@@ -977,6 +998,7 @@ static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
   const int64_t nt = Y.nrows * 32;
   TX* X = (TX*)x->d_lx;
   TX* XT = (TX*)x->d_lxt;
+  // in full: the launches behind it read the system before their waits
   dev::k_lsgs_init<<<1, 1, 0, s>>>(ctl, x->P.lsgs_relaxation);
   int rc;
   if (jacobi_start && (rc = launch_thomas<TB, TD, TX>(x, 0, Y.ngroups, true, nullptr))) return rc;
@@ -991,15 +1013,15 @@ static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
         const int64_t rb = Y.grp_row0[g0];
         const int64_t re = Y.grp_row0[g0 + ng - 1] + Y.grp_len[g0 + ng - 1];
         prof_begin(x, "lsgs_rhs");
-        dev::k_lsgs_rhs<TB, TX><<<nblocks((re - rb) * 32, 128), 128, 0, s>>>(
+        launch_chain(x, dev::k_lsgs_rhs<TB, TX>, nblocks((re - rb) * 32, 128), 128, 0,
             rb, re - rb, V, (const TB*)x->d_lF, (const TB*)x->d_lB, X, (TX*)x->d_lrhs,
             pass == 1 ? XT : nullptr, ctl);
         prof_end(x);
         if ((rc = launch_thomas<TB, TD, TX>(x, g0, ng, false, ctl))) return rc;
       }
     prof_begin(x, "lsgs_relax");
-    dev::k_lsgs_relax<TX><<<nblk, dev::RELAX_THREADS, 0, s>>>(nt, X, XT, ctl, x->d_lpart);
-    dev::k_lsgs_control<<<1, dev::RELAX_THREADS, 0, s>>>(x->d_lpart, nblk, x->P.lsgs_abs_tol,
+    launch_chain(x, dev::k_lsgs_relax<TX>, nblk, dev::RELAX_THREADS, 0, nt, X, XT, ctl, x->d_lpart);
+    launch_chain(x, dev::k_lsgs_control, 1, dev::RELAX_THREADS, 0, x->d_lpart, nblk, x->P.lsgs_abs_tol,
                                                          x->P.lsgs_rel_tol, ctl);
     prof_end(x);
   }
