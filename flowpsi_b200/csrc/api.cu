@@ -515,7 +515,8 @@ int fpsi_create(fpsi_ctx** out, const fpsi_mesh* mesh, const fpsi_params* params
     return FPSI_E_CUDA;
   }
   x->nblk_norm = int((nc + 255) / 256);
-  TRY(dalloc(x, &x->d_part, size_t(x->nblk_norm) * 8));
+  // norms: 8 per 256 cells; linear residual: 2 per 128 cells of a colour
+  TRY(dalloc(x, &x->d_part, size_t(x->nblk_norm) * 8 + 2 * size_t(H.ncolours)));
   TRY(dalloc(x, &x->d_resid, 32));
   TRY(dalloc(x, &x->d_amin, size_t(x->nblk_norm)));
   TRY(dalloc(x, &x->d_err, 4));

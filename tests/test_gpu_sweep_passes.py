@@ -84,3 +84,34 @@ def test_sweeps_match_oracle(need_gpu, name, prec):
             e_orc, e_gpu = (np.abs(d[:, k] - d64[:, k]).max() for d in (do, dg))
             assert e_gpu <= 2.0 * e_orc + 1e-6 * np.abs(d64[:, k]).max(), k
     g.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "ref", "mixed"])
+@pytest.mark.parametrize("name", [n for n in CASES if n != "hex_49"])
+def test_linear_residual_is_that_of_the_exported_blocks(need_gpu, name, prec):
+    """||B|| and ||B - A x|| from the sweeps' slots against the exported
+    blocks in FP64: the same entries, sums of some 1e3 terms in another order
+    (1e-13 relative each), so 1e-11 of ||B|| + sum |A| |x|"""
+    case, st, _ = _dq(name, prec)
+    g = FlowPsi(case.mesh, case.params)
+    g.set_state(*st)
+    g.residual()
+    g.assemble()
+    g.sweeps(2)
+    nb, nr = g.linear_residual()
+    x, b = g.get_iterate(), {k: v.astype(np.float64) for k, v in g.blocks().items()}
+    a = case.mesh.arrays() if hasattr(case.mesh, "arrays") else case.pairs
+    inner = np.flatnonzero(np.asarray(a.cr) >= 0)
+    cl, cr = np.asarray(a.cl)[inner], np.asarray(a.cr)[inner]
+
+    def apply(D, fjp, fjm, v):
+        y = np.einsum("cij,cj->ci", D, v)
+        np.add.at(y, cl, np.einsum("fij,fj->fi", fjm, v[cr]))
+        np.add.at(y, cr, np.einsum("fij,fj->fi", fjp, v[cl]))
+        return y
+
+    r = b["fluid_B"] - apply(b["fluid_D"], -b["fjp"][inner], b["fjm"][inner], x)
+    size = np.linalg.norm(apply(*(np.abs(m) for m in (b["fluid_D"], b["fjp"][inner], b["fjm"][inner], x))))
+    assert abs(nb - np.linalg.norm(b["fluid_B"])) <= 1e-11 * nb
+    assert abs(nr - np.linalg.norm(r)) <= 1e-11 * (nb + size)
+    g.close()
