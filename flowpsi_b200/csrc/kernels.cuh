@@ -14,6 +14,10 @@ int launch_residual(fpsi_ctx* x, double* resid_slot);
 // the gradient-and-limiter records of the last residual's state (written
 // by the residual itself only for viscous runs)
 int launch_grad_records(fpsi_ctx* x);
+// the cells' viscosity and conductivity, for the last residual's state and the
+// options in force (the residual of a viscous run leaves them; options may
+// have changed since)
+int ensure_material(fpsi_ctx* x);
 // face Jacobians, diagonal blocks, LU, B and the starting iterate
 // (the starting iterate is the block Jacobi start D^-1 B)
 int launch_assemble(fpsi_ctx* x);

@@ -43,6 +43,7 @@ struct Geo {
 
 struct Gas {
   double gamma, Rt, pamb, a1, a2, a3;
+  const double* muk;  // [nc][2]: the cells' Sutherland viscosity (and conductivity), from the residual
 };
 
 __device__ __forceinline__ double suth(double T, const Gas& g) {
@@ -183,7 +184,7 @@ __global__ void k_sa_face(Geo G, const double* q, const double* qb,
     const double vl = G.vol[a], vr = G.vol[b];
     const double rho_b = rho_of(q, b, g);
     const double nuf = (vr * nut[a] + vl * nut[b]) * (1.0 / (vr + vl));
-    const double muf = (vl * suth(q[5 * b], g) + vr * suth(q[5 * a], g)) / (vl + vr);
+    const double muf = (vl * g.muk[2 * b] + vr * g.muk[2 * a]) / (vl + vr);
     const double rhof = (1. / (vl + vr)) * (vl * rho_b + vr * rho_a);
     const double d0 = rl0 - rr0, d1 = rl1 - rr1, d2 = rl2 - rr2;
     const double dsq = d0 * d0 + d1 * d1 + d2 * d2;
@@ -284,7 +285,7 @@ __global__ void k_sa_cell(Geo G, const double* q, const double* grad,
     }
   }
   const double nu = nut[c], V = G.vol[c], y = wdist[c];
-  const double mu = suth(q[5 * c], g);
+  const double mu = g.muk[2 * c];
   const double* gu = grad + GPREC * c + 3;  // rows u, v, w: d u_i / d x_j
   const double wx = gu[3 * 2 + 1] - gu[3 * 1 + 2];
   const double wy = gu[3 * 0 + 2] - gu[3 * 2 + 0];
@@ -434,7 +435,7 @@ sa::Geo geo(const fpsi_ctx* x) {
   return G;
 }
 sa::Gas sgas(const fpsi_ctx* x) {
-  return sa::Gas{x->P.gamma, x->P.Rtilde, x->P.Pambient, x->P.mu_a1, x->P.mu_a2, x->P.mu_a3};
+  return sa::Gas{x->P.gamma, x->P.Rtilde, x->P.Pambient, x->P.mu_a1, x->P.mu_a2, x->P.mu_a3, x->d_muk};
 }
 }  // namespace
 
@@ -452,6 +453,8 @@ int sa_launch_tmu(fpsi_ctx* x) {
 }
 
 int sa_launch_residual(fpsi_ctx* x) {
+  const int rc = ensure_material(x);
+  if (rc) return rc;
   const sa::Geo G = geo(x);
   const sa::Gas g = sgas(x);
   prof_begin(x, "sa_grad");
