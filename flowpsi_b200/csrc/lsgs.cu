@@ -309,11 +309,11 @@ __device__ __forceinline__ T quotient(T a, T b, T y) {
   const T q = fma(a, y, a * yl);
   return fma(fma(-b, q, a), y, q);
 }
-// |b| in 2^-36 .. 2^28 (FP32), 2^-300 .. 2^300 (FP64)
-__device__ __forceinline__ bool pivot_ok(float b) { return fabsf(b) >= 0x1p-36f && fabsf(b) <= 0x1p28f; }
+// |b| in 2^-100 .. 2^28 (FP32), 2^-300 .. 2^300 (FP64)
+__device__ __forceinline__ bool pivot_ok(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p28f; }
 __device__ __forceinline__ bool pivot_ok(double b) { return fabs(b) >= 0x1p-300 && fabs(b) <= 0x1p300; }
 // the smallest nonzero |a| so far, as a key (twice its bits, less one; zero
-// gives the largest key), and whether one below 2^-74 (2^-600) was among
+// gives the largest key), and whether one below 2^-90 (2^-600) was among
 // them: there the remainder or the reciprocal's second part may underflow.
 // Above, an overflow ends in a NaN.
 __device__ __forceinline__ uint32_t key_min(uint32_t k, float a) { return min(k, 2u * __float_as_uint(a) - 1u); }
@@ -322,7 +322,7 @@ __device__ __forceinline__ uint32_t key_min(uint32_t k, double a) {
 }
 template <class T>
 __device__ __forceinline__ bool tiny(uint32_t k) {
-  return k < (sizeof(T) == 4 ? 2u * ((127u - 74u) << 23) : 2u * ((1023u - 600u) << 20)) - 1u;
+  return k < (sizeof(T) == 4 ? 2u * ((127u - 90u) << 23) : 2u * ((1023u - 600u) << 20)) - 1u;
 }
 
 // Gather the line-ordered system: raw diagonal block, in-line couplings
@@ -419,10 +419,36 @@ __device__ __forceinline__ void lu5_recip_solve(const T* A, const T* r, T* y, ui
   }
 }
 
+// lu5_nopiv that also gives the pivots' reciprocals r[5] (NaN outside the
+// range of quotient()); key: of the dividends
+template <class T>
+__device__ __forceinline__ void lu5_nopiv_recip(T* A, T* r, uint32_t& key) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const T d = A[6 * k];
+    r[k] = pivot_ok(d) ? T(1) / d : T(nanf(""));
+#pragma unroll
+    for (int i = k + 1; i < 5; ++i) {
+      key = key_min(key, A[5 * i + k]);
+      A[5 * i + k] = quotient<T>(A[5 * i + k], d, r[k]);
+#pragma unroll
+      for (int j = k + 1; j < 5; ++j) A[5 * i + j] -= A[5 * i + k] * A[5 * k + j];
+    }
+  }
+}
+
 // block Thomas preprocessing (preprocessLine, linearSolverLSGS.loci:1465-1495):
 // D'_0 = D_0, D'_p = D_p - L_p D'_{p-1}^{-1} U_{p-1}; each D' factored in
 // place.  As in the reference the Schur product is formed with real_fj
 // (TB) intermediates.
+//
+// A serial chain per line with less than a warp per SM, so a row's
+// instructions set it, and most of them were its 40 divisions.  Five remain
+// (the pivots' reciprocals, which the solves need as well); the others are
+// quotient()s.  A row whose operands leave their range, or that comes out
+// not finite, is done again with divisions.  262,144 cells in rows of 64:
+// 134 -> 70 us MIXED; 24,576 cells in rows of 32: 114 -> 76 us REF, 109 -> 82 us
+// FP64 (whose next row's blocks do not fit beside this one's).
 template <class TB, class TD>
 __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
                             const TB* lL, const TB* lU,
@@ -434,39 +460,82 @@ __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
   const int64_t g = gl >> 5, lane = gl & 31;
   const int len = V.lane_len[gl];
   const int64_t r0 = V.grp_row0[g];
-  TD prev[25];
-  for (int p = 0; p < len; ++p) {
+  TD prev[25], rp[5];  // the row before: its factors and their pivots' reciprocals
+  constexpr bool AHEAD = sizeof(TD) == 4;  // the next row's blocks fit in registers
+  struct Blocks {
+    TD D[25];
+    TB L[25], U[25];
+  } nx;
+  auto load = [&](int p, Blocks& w) {
     const int64_t r = r0 + p;
-    TD Dp[25];
-    block_load<TD>(lD + r * DROW, int(lane), Dp);
+    block_load<TD>(lD + r * DROW, int(lane), w.D);
     if (p > 0) {
-      TB Lm[25], Um[25];
-      block_load<TB>(lL + r * 25 * 32, int(lane), Lm);
-      block_load<TB>(lU + (r - 1) * 25 * 32, int(lane), Um);
+      block_load<TB>(lL + r * 25 * 32, int(lane), w.L);
+      block_load<TB>(lU + (r - 1) * 25 * 32, int(lane), w.U);
+    }
+  };
+  // row p from its blocks; whether the result stands
+  auto row = [&](int p, Blocks& w, bool exact, TD* rn) {
+    TD* Dp = w.D;
+    uint32_t key = ~0u;
+    TD chk = TD(0);  // stays 0 while everything is finite
+    if (p > 0) {
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
         TD v[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) v[k] = TD(Um[5 * k + j]);
-        lu5_nopiv_solve<TD, TD>(prev, v);
-        TB tt[5], w[5];
+        for (int k = 0; k < 5; ++k) v[k] = TD(w.U[5 * k + j]);
+        if (exact)
+          lu5_nopiv_solve<TD, TD>(prev, v);
+        else
+          lu5_recip_solve<TD>(prev, rp, v, key);
+        TB tt[5], z[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) tt[k] = TB(v[k]), w[k] = TB(0);
+        for (int k = 0; k < 5; ++k) chk += v[k] * TD(0), tt[k] = TB(v[k]), z[k] = TB(0);
 #pragma unroll
         for (int k = 0; k < 5; ++k)
 #pragma unroll
-          for (int m = 0; m < 5; ++m) w[k] += Lm[5 * k + m] * tt[m];
+          for (int m = 0; m < 5; ++m) z[k] += w.L[5 * k + m] * tt[m];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) Dp[5 * k + j] -= TD(w[k]);
+        for (int k = 0; k < 5; ++k) Dp[5 * k + j] -= TD(z[k]);
       }
     }
-    if (!lu5_nopiv<TD>(Dp)) atomicOr(err, 2);
-    block_store<TD>(lD + r * DROW, int(lane), Dp);
+    if (exact) {
+      if (!lu5_nopiv<TD>(Dp)) atomicOr(err, 2);
 #pragma unroll
-    for (int k = 0; k < 5; ++k)
-      lD[r * DROW + (25 + k) * 32 + lane] = pivot_ok(Dp[6 * k]) ? TD(1) / Dp[6 * k] : TD(nanf(""));
+      for (int k = 0; k < 5; ++k) rn[k] = pivot_ok(Dp[6 * k]) ? TD(1) / Dp[6 * k] : TD(nanf(""));
+      return true;
+    }
+    lu5_nopiv_recip<TD>(Dp, rn, key);
 #pragma unroll
-    for (int e = 0; e < 25; ++e) prev[e] = Dp[e];
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int i = k + 1; i < 5; ++i) chk += Dp[5 * i + k] * TD(0);
+    // the last pivot divides nothing in its own row but must not be zero
+    return chk == TD(0) && !tiny<TD>(key) && Dp[24] != TD(0);
+  };
+  if (AHEAD && len > 0) load(0, nx);
+  for (int p = 0; p < len; ++p) {
+    const int64_t r = r0 + p;
+    Blocks w;
+    if (AHEAD) {
+      w = nx;
+      if (p + 1 < len) load(p + 1, nx);
+    } else {
+      load(p, w);
+    }
+    TD rn[5];
+    if (!row(p, w, false, rn)) {
+      load(p, w);  // its own block is still the raw one
+      row(p, w, true, rn);
+    }
+    block_store<TD>(lD + r * DROW, int(lane), w.D);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) lD[r * DROW + (25 + k) * 32 + lane] = rn[k];
+#pragma unroll
+    for (int e = 0; e < 25; ++e) prev[e] = w.D[e];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) rp[k] = rn[k];
   }
 }
 

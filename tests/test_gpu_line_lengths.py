@@ -87,3 +87,34 @@ def test_zero_right_hand_side_stays_zero(need_gpu, prec):
     assert np.isfinite(dq).all()
     assert np.abs(dq[:, 0]).max() <= 1e-6 and np.abs(dq[:, 4]).max() <= 1e-3  # of 300 K, 1e5 Pa
     g.close()
+
+
+@pytest.mark.parametrize("prec", ["ref", "mixed"])
+@pytest.mark.parametrize("size", [1e-16, 1e-15, 1e-7])
+def test_small_domains_match_oracle(need_gpu, size, prec):
+    """areas so small that the FP32 blocks' pivots lie below the range of the
+    stored reciprocals (2^-100; most of them, some, none): the factoring and
+    the solves take their divisions there.  Bars as above."""
+    def mk(p):
+        mesh, c = _case(9, p)
+        U0 = 0.5 * np.sqrt(cases.GAMMA * cases.RTILDE * 300.0)
+        return GeneratedMesh("hex", n=(5, 9, 3), L=(size, 1.8 * size, 0.6 * size), bc_side=(0,) * 6,
+                             bcs=[bc("farfield", u=(U0, 0.0, 0.0))]), c
+
+    mesh, c = mk(prec)
+    g = FlowPsi(mesh, c.params)
+    g.set_lines(mesh.lines_along(1))
+    lines, colours = g.line_list()
+    o, o64 = Oracle(mesh, c.params), Oracle(*(lambda m, k: (m, k.params))(*mk("fp64")))
+    cc = o.geometry()["cellcenter"] / size
+    state = (300.0 + 20.0 * np.sin(5 * cc[:, 0]), 1e5 + 5e3 * np.cos(4 * cc[:, 1]),
+             50.0 + 30.0 * np.sin(3 * cc + [0.0, 1.0, 2.0]))
+    for s in (g, o, o64):
+        s.set_state(*state)
+        s.residual()
+        s.assemble()
+    dg, do, d64 = g.linear_solve(), o.lsgs_solve(lines, colours)[0], o64.lsgs_solve(lines, colours)[0]
+    for k in range(5):
+        e_orc, e_gpu = (np.abs(d[:, k] - d64[:, k]).max() for d in (do, dg))
+        assert e_gpu <= 2.0 * e_orc + 1e-6 * np.abs(d64[:, k]).max(), k
+    g.close()

@@ -43,3 +43,14 @@ def test_quotient_is_correctly_rounded(seed):
         b = draw(r, -36, 27)
         a = r.choice([draw(r, -74, 80), draw(r, -74, -70), rn(draw(r, -30, 30) * b)])
         assert quotient(a, b) == rn(a / b), (a, b)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_quotient_of_small_operands(seed):
+    """pivots down to 2^-100, dividends down to 2^-90"""
+    r = random.Random(100 + seed)
+    for _ in range(4000):
+        b = draw(r, *r.choice([(-100, 27), (-100, -98), (26, 27)]))
+        a = r.choice([draw(r, -90, 20), draw(r, -90, -88), rn(draw(r, -20, 20) * b)])
+        if abs(a) >= Fraction(1, 2**90) and abs(a / b) < 2**120:  # overflow ends in a NaN
+            assert quotient(a, b) == rn(a / b), (a, b)
