@@ -193,19 +193,12 @@ int alloc_lsgs(fpsi_ctx* x) {
   return FPSI_OK;
 }
 
-// residual history for runs of up to n steps (8 doubles per step)
+// residual history for runs of up to n steps
 int ensure_hist(fpsi_ctx* x, int64_t n) {
   if (n <= x->hist_cap) return FPSI_OK;
-  if (x->d_hist) {
-    x->device_bytes -= x->hist_cap * fpsi::NREC * int64_t(sizeof(double));
-    cudaFree(x->d_hist);
-    x->d_hist = nullptr;
-  }
   if (x->h_hist) cudaFreeHost(x->h_hist);
   x->h_hist = nullptr;
   x->hist_cap = 0;
-  int rc = dalloc(x, &x->d_hist, size_t(n) * fpsi::NREC);
-  if (rc) return rc;
   if (cudaMallocHost((void**)&x->h_hist, size_t(n) * fpsi::NREC * sizeof(double)) != cudaSuccess) {
     fpsi::set_error("cudaMallocHost of the residual history failed");
     return FPSI_E_NOMEM;
@@ -397,7 +390,6 @@ int fpsi_destroy(fpsi_ctx* x) {
   if (x->h_resid) cudaFreeHost(x->h_resid);
   if (x->h_flags) cudaFreeHost(x->h_flags);
   if (x->h_amin) cudaFreeHost(x->h_amin);
-  if (x->d_hist) cudaFree(x->d_hist);
   if (x->h_hist) cudaFreeHost(x->h_hist);
   for (cudaEvent_t e : x->evpool) cudaEventDestroy(e);
   if (x->stream) cudaStreamDestroy(x->stream);
@@ -1018,9 +1010,9 @@ int fpsi_newton_step(fpsi_ctx* x, fpsi_stepinfo* info) {
   int rc;
   const bool sa = fpsi::sa_active(x);
   if (sa && (rc = fpsi::sa_launch_tmu(x))) return rc;
-  if ((rc = fpsi::launch_residual(x, x->d_resid))) return rc;
+  if ((rc = fpsi::launch_residual(x, nullptr))) return rc;
   if (sa && ((rc = fpsi::sa_launch_residual(x)) || (rc = fpsi::sa_launch_solve(x)))) return rc;
-  if ((rc = fpsi::launch_assemble(x))) return rc;
+  if ((rc = fpsi::launch_assemble(x, {x->d_resid, x->h_resid, nullptr}))) return rc;
   if (is_lsgs(x)) {
     if ((rc = fpsi::lsgs_assemble(x))) return rc;
     if ((rc = fpsi::lsgs_solve(x, true))) return rc;
@@ -1029,8 +1021,6 @@ int fpsi_newton_step(fpsi_ctx* x, fpsi_stepinfo* info) {
   }
   if ((rc = fpsi::launch_update(x, x->d_resid))) return rc;
   if (sa && (rc = fpsi::sa_launch_update(x, x->d_resid))) return rc;
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid, x->d_resid, fpsi::NREC * sizeof(double),
-                                cudaMemcpyDeviceToHost, x->stream));
   std::vector<double> a(x->nblk_norm);
   FPSI_CUDA_TRY(cudaMemcpyAsync(a.data(), x->d_amin, a.size() * sizeof(double),
                                 cudaMemcpyDeviceToHost, x->stream));
@@ -1209,41 +1199,35 @@ int fpsi_newton_step_ex(fpsi_ctx* x, fpsi_gnn* model, const fpsi_step_opts* opts
   return FPSI_OK;
 }
 
-// One implicit step's launches on the stream, its norms into slot (device)
-// and, when hdst is given, by a copy queued behind the residual into hdst
-// (pinned host).
-static int launch_step(fpsi_ctx* x, double* slot, double* hdst, bool sa) {
+// One implicit step's launches on the stream; its norms go to d_resid and to
+// the history's next record.
+static int launch_step(fpsi_ctx* x, bool sa) {
   int rc = FPSI_OK;
   if (sa) rc = fpsi::sa_launch_tmu(x);
-  if (!rc) rc = fpsi::launch_residual(x, slot);
-  if (!rc && hdst &&
-      cudaMemcpyAsync(hdst, slot, fpsi::NREC * sizeof(double), cudaMemcpyDeviceToHost, x->stream) !=
-          cudaSuccess)
-    rc = FPSI_E_CUDA;
+  if (!rc) rc = fpsi::launch_residual(x, nullptr);
   if (!rc && sa) rc = fpsi::sa_launch_residual(x);
   if (!rc && sa) rc = fpsi::sa_launch_solve(x);
-  if (!rc) rc = fpsi::launch_assemble(x);
+  if (!rc) rc = fpsi::launch_assemble(x, {x->d_resid, x->h_hist, x->d_err + 2});
   if (!rc && is_lsgs(x)) {
     rc = fpsi::lsgs_assemble(x);
     if (!rc) rc = fpsi::lsgs_solve(x, true);
   } else if (!rc) {
     rc = fpsi::launch_sgs(x, x->P.gauss_seidel_iter);
   }
-  if (!rc) rc = fpsi::launch_update(x, slot);
-  if (!rc && sa) rc = fpsi::sa_launch_update(x, slot);
+  if (!rc) rc = fpsi::launch_update(x, x->d_resid);
+  if (!rc && sa) rc = fpsi::sa_launch_update(x, x->d_resid);
   return rc;
 }
 
-// The launches of one step captured as a CUDA graph, with its norms going to
-// the fixed slot; null when the capture or the instantiation fails (the
+// The launches of one step captured as a CUDA graph; null when the capture or the instantiation fails (the
 // caller then launches the step itself).  Nothing of a captured step runs
 // until the graph is launched.
-static cudaGraphExec_t capture_step(fpsi_ctx* x, double* fixed) {
+static cudaGraphExec_t capture_step(fpsi_ctx* x) {
   if (cudaStreamBeginCapture(x->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  const int rc = launch_step(x, fixed, nullptr, fpsi::sa_active(x));
+  const int rc = launch_step(x, fpsi::sa_active(x));
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(x->stream, &g);
   cudaGraphExec_t ge = nullptr;
@@ -1257,25 +1241,24 @@ static cudaGraphExec_t capture_step(fpsi_ctx* x, double* fixed) {
 
 // nsteps implicit steps on the stream; with the SA model nu~ is advanced in
 // each step from the same residual state, after the mean flow's solve.  The
-// norms of step s go to d_hist[NREC s] and, by a copy queued behind the
-// residual, to the pinned h_hist[NREC s] (whose rtrms slot starts at -1).
-// Before each launch the host looks at the copies that have landed and stops
+// step's kernel that finishes its norms writes them straight to the pinned
+// h_hist[NREC s] (whose rtrms slot starts at -1), s counted on the device, so
+// that a step is its kernels alone, the same for each step.
+// Before each launch the host looks at the records that have landed and stops
 // launching once one holds NaN norms; steps already queued behind it leave
 // the state alone (the update kernels test their step's norms), so the state
 // is the one of the first NaN step.  With step_graphs step 0 runs as
-// launches, which makes every buffer the step uses, and steps
-// 1.. replay one captured graph whose norms land in d_hist[NREC nsteps]
-// (the history holds nsteps + 1 records) and are copied from there into
-// the step's slots behind the graph.
+// launches, which makes every buffer the step uses, and steps 1.. replay one
+// captured graph.
 // Returns the number of steps launched.
 static int run_steps(fpsi_ctx* x, int32_t nsteps, int32_t* launched) {
   int rc = FPSI_OK;
   const bool sa = fpsi::sa_active(x);
   const bool graphs = x->P.step_graphs && !x->profiling && nsteps > 2;
-  double* fixed = x->d_hist + fpsi::NREC * int64_t(nsteps);
   cudaGraphExec_t ge = nullptr;
   volatile double* hh = x->h_hist;
   for (int32_t s = 0; s < nsteps; ++s) hh[fpsi::NREC * int64_t(s)] = -1.0;
+  if (cudaMemsetAsync(x->d_err + 2, 0, sizeof(int32_t), x->stream) != cudaSuccess) return FPSI_E_CUDA;
   int32_t seen = 0, s = 0;
   for (; s < nsteps && !rc; ++s) {
     bool nan = false;
@@ -1287,19 +1270,11 @@ static int run_steps(fpsi_ctx* x, int32_t nsteps, int32_t* launched) {
       ++seen;
     }
     if (nan) break;
-    double* slot = x->d_hist + fpsi::NREC * int64_t(s);
-    double* hdst = x->h_hist + fpsi::NREC * int64_t(s);
-    if (graphs && s == 1) ge = capture_step(x, fixed);
-    if (ge) {
-      if (cudaGraphLaunch(ge, x->stream) != cudaSuccess ||
-          cudaMemcpyAsync(slot, fixed, fpsi::NREC * sizeof(double), cudaMemcpyDeviceToDevice,
-                          x->stream) != cudaSuccess ||
-          cudaMemcpyAsync(hdst, fixed, fpsi::NREC * sizeof(double), cudaMemcpyDeviceToHost,
-                          x->stream) != cudaSuccess)
-        rc = FPSI_E_CUDA;
-    } else {
-      rc = launch_step(x, slot, hdst, sa);
-    }
+    if (graphs && s == 1) ge = capture_step(x);
+    if (!ge)
+      rc = launch_step(x, sa);
+    else if (cudaGraphLaunch(ge, x->stream) != cudaSuccess)
+      rc = FPSI_E_CUDA;
   }
   if (ge) cudaGraphExecDestroy(ge);
   *launched = s;
@@ -1336,7 +1311,7 @@ static int finish_run(fpsi_ctx* x, int32_t nsteps, int32_t launched, fpsi_resid*
 int fpsi_run(fpsi_ctx* x, int32_t nsteps, fpsi_resid* norms) {
   if (!x || nsteps < 0) return FPSI_E_INVALID;
   if (nsteps == 0) return FPSI_OK;
-  int rc = ensure_hist(x, nsteps + 1);
+  int rc = ensure_hist(x, nsteps);
   if (rc) return rc;
   int32_t launched = 0;
   rc = run_steps(x, nsteps, &launched);
@@ -1353,7 +1328,7 @@ int fpsi_time_step(fpsi_ctx* x, fpsi_resid* norms) {
     return FPSI_E_STATE;
   }
   const int32_t nit = x->P.newton_iters;
-  int rc = ensure_hist(x, nit + 1);
+  int rc = ensure_hist(x, nit);
   if (rc) return rc;
   int32_t launched = 0;
   rc = run_steps(x, nit, &launched);
@@ -1370,7 +1345,7 @@ int fpsi_time_step(fpsi_ctx* x, fpsi_resid* norms) {
 
 int fpsi_run_timed(fpsi_ctx* x, int32_t nsteps, fpsi_resid* norms, double* device_ms) {
   if (!x || nsteps <= 0 || !device_ms) return FPSI_E_INVALID;
-  int rc = ensure_hist(x, nsteps + 1);
+  int rc = ensure_hist(x, nsteps);
   if (rc) return rc;
   cudaEvent_t a = nullptr, b = nullptr;
   if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) rc = FPSI_E_CUDA;
@@ -1392,7 +1367,7 @@ int fpsi_run_timed(fpsi_ctx* x, int32_t nsteps, fpsi_resid* norms, double* devic
 int fpsi_kernel_times(fpsi_ctx* x, int32_t nsteps, int32_t cap, char* names, double* ms,
                       int64_t* launches, int32_t* count) {
   if (!x || nsteps <= 0 || cap < 0 || !count) return FPSI_E_INVALID;
-  int rc = ensure_hist(x, nsteps + 1);
+  int rc = ensure_hist(x, nsteps);
   if (rc) return rc;
   x->prof.clear();
   x->evnext = 0;

@@ -174,10 +174,9 @@ struct fpsi_ctx {
   // the update's per-block step fractions, read after its one synchronisation
   int32_t* h_flags = nullptr;
   double* h_amin = nullptr;
-  // residual history of fpsi_run / fpsi_run_timed: 8 norms per step on the
-  // device and their pinned host mirror, kept for the context's life (grown
+  // residual history of fpsi_run / fpsi_run_timed: NREC values per step in
+  // pinned memory that the steps write, kept for the context's life (grown
   // only for a longer run than any before)
-  double* d_hist = nullptr;
   double* h_hist = nullptr;
   int64_t hist_cap = 0;
   // state copy of fpsi_newton_step_ex, to undo a rejected update
@@ -205,7 +204,8 @@ struct fpsi_ctx {
   fpsi::ColInfo* d_colinfo = nullptr;
   void* d_x = nullptr;         // [nc][5] TX, colour order
   double* d_amin = nullptr;    // per-block min alpha
-  int32_t* d_err = nullptr;    // error flags (singular pivots, ...)
+  int32_t* d_err = nullptr;    // [0] error flags (singular pivots, ...), [1] boundary conditions' bits,
+                               // [2] steps of the run whose norms are written
   int blk_bytes = 4;           // sizeof(TB)
   int x_bytes = 8;             // sizeof(TX)
   int alloc_prec = -1;

@@ -944,6 +944,14 @@ k_alpha_diss(MeshView M, const double* __restrict__ q, const double* __restrict_
 // per-cell residual gather, local time step and norm partials
 // ---------------------------------------------------------------------------
 constexpr int NORM_THREADS = 256;
+// the last residual's partial norms (null part: none to finish) and where
+// their result goes
+struct NormSink {
+  const double* part;
+  int nblk;
+  int32_t* bcflags;
+  NormOut to;
+};
 
 template <bool BDF>
 __global__ void __launch_bounds__(NORM_THREADS)
@@ -1103,23 +1111,38 @@ k_cell_residual(MeshView M, const double* __restrict__ q, const double* __restri
   }
 }
 
-// out[0..2] = rms (sqrt of sums), out[3..4] rtmax/loc, out[5..6] etmax/loc,
-// out[7] mtmax; written to slot `step` of a per-run history
-__global__ void k_norm_final(const double* __restrict__ part, int nblk,
-                             int32_t* __restrict__ bcflags, double* __restrict__ out) {
-  __shared__ double sh[8][NORM_THREADS];
+// The norms from the blocks' partials: out[0..2] = rms (sqrt of sums),
+// out[3..4] rtmax/loc, out[5..6] etmax/loc, out[7] mtmax, out[8] the
+// boundary-condition error bits of this residual (cleared for the next).
+// One block of T threads, the partials in NORM_THREADS chains whatever T is;
+// sh: its shared memory.  With a host record (pinned memory, of a run's step
+// *seq where seq is given) they are written there as well, the first entry
+// last, so that a host that polls it finds the others.
+//
+// A chain of a few us that nothing before the update reads: a step has its
+// assembly's first block do it beside the others (k_norm_final, in the
+// stream between two kernels, where there is no assembly).  A run's step
+// that left its norms to k_norm_final and two 80 B copies behind the step's
+// graph took 20 us more: 32,768 hexes REF 0.121 -> 0.102 ms a step, 24,576
+// tets MIXED 0.165 -> 0.147, 262,144 cells with lines and SA 2.05 -> 2.01.
+template <int T>
+__device__ __forceinline__ void norm_final(const NormSink& N, double (*sh)[NORM_THREADS]) {
   const int t = threadIdx.x;
-  double a[8] = {0, 0, 0, 0, -1, 0, -1, 0};
-  for (int i = t; i < nblk; i += NORM_THREADS) {
-    const double* p = part + 8 * int64_t(i);
-    a[0] += p[0], a[1] += p[1], a[2] += p[2];
-    if (fabs(p[3]) > fabs(a[3]) || (fabs(p[3]) == fabs(a[3]) && a[4] < 0)) a[3] = p[3], a[4] = p[4];
-    if (fabs(p[5]) > fabs(a[5]) || (fabs(p[5]) == fabs(a[5]) && a[6] < 0)) a[5] = p[5], a[6] = p[6];
-    if (fabs(p[7]) > fabs(a[7])) a[7] = p[7];
-  }
+#pragma unroll 1
+  for (int v = t; v < NORM_THREADS; v += T) {
+    double a[8] = {0, 0, 0, 0, -1, 0, -1, 0};
+    for (int i = v; i < N.nblk; i += NORM_THREADS) {
+      const double* p = N.part + 8 * int64_t(i);
+      a[0] += p[0], a[1] += p[1], a[2] += p[2];
+      if (fabs(p[3]) > fabs(a[3]) || (fabs(p[3]) == fabs(a[3]) && a[4] < 0)) a[3] = p[3], a[4] = p[4];
+      if (fabs(p[5]) > fabs(a[5]) || (fabs(p[5]) == fabs(a[5]) && a[6] < 0)) a[5] = p[5], a[6] = p[6];
+      if (fabs(p[7]) > fabs(a[7])) a[7] = p[7];
+    }
 #pragma unroll
-  for (int k = 0; k < 8; ++k) sh[k][t] = a[k];
+    for (int k = 0; k < 8; ++k) sh[k][v] = a[k];
+  }
   __syncthreads();
+#pragma unroll 1
   for (int st = NORM_THREADS / 2; st > 0; st >>= 1) {
     if (t < st) {
       sh[0][t] += sh[0][t + st];
@@ -1142,16 +1165,28 @@ __global__ void k_norm_final(const double* __restrict__ part, int nblk,
     __syncthreads();
   }
   if (t == 0) {
-    out[0] = sqrt(sh[0][0]);
-    out[1] = sqrt(sh[1][0]);
-    out[2] = sqrt(sh[2][0]);
+    double r[NREC];
 #pragma unroll
-    for (int k = 3; k < 8; ++k) out[k] = sh[k][0];
-    // the boundary-condition error bits of this residual, cleared for the next
-    out[8] = double(*bcflags);
-    out[9] = 0.0;
-    *bcflags = 0;
+    for (int k = 0; k < 8; ++k) r[k] = k < 3 ? sqrt(sh[k][0]) : sh[k][0];
+    r[8] = double(*N.bcflags);
+    r[9] = 0.0;
+    *N.bcflags = 0;
+#pragma unroll
+    for (int k = 0; k < NREC; ++k) N.to.rec[k] = r[k];
+    if (N.to.host) {
+      int64_t s = 0;
+      if (N.to.seq) s = (*N.to.seq)++;
+      volatile double* h = N.to.host + NREC * s;
+#pragma unroll
+      for (int k = 1; k < NREC; ++k) h[k] = r[k];
+      __threadfence_system();
+      h[0] = r[0];
+    }
   }
+}
+__global__ void __launch_bounds__(NORM_THREADS) k_norm_final(NormSink N) {
+  __shared__ double sh[8][NORM_THREADS];
+  norm_final<NORM_THREADS>(N, sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -1506,16 +1541,21 @@ k_assemble(MeshView M, SweepView S, const double* __restrict__ q, const double* 
            const double* __restrict__ dtau, const TB* __restrict__ fjp, const TB* __restrict__ fjm,
            const TB* __restrict__ fjc, Gas g, TB* __restrict__ luc, TB* __restrict__ bcv,
            int32_t* __restrict__ pvv, TB* __restrict__ aoff, TB* __restrict__ Dout, TX* __restrict__ x,
-           int32_t* __restrict__ err, double dcoef, const TB* __restrict__ bjac) {
+           int32_t* __restrict__ err, double dcoef, const TB* __restrict__ bjac, NormSink N) {
   constexpr int RW = 50;  // words staged per face (explicit blocks)
   constexpr int U16 = asm_u16<TB>(), RS16 = asm_rs16<TB>();
   static_assert(CK_FACE * sizeof(TB) % 16 == 0, "a compact record is whole 16 B units");
   static_assert(32 * 25 * sizeof(TB) <= asm_warp_bytes<TB, CPT>(), "the diagonal blocks fit the staging area");
+  static_assert(8 * NORM_THREADS * sizeof(double) <= asm_smem_bytes<TB, CPT>(), "the norms' chains fit it too");
   extern __shared__ __align__(16) unsigned char asm_smem[];
+  if (N.part && blockIdx.x == 0) {
+    norm_final<ASM_THREADS>(N, reinterpret_cast<double(*)[NORM_THREADS]>(asm_smem));
+    return;
+  }
   TB* st = reinterpret_cast<TB*>(asm_smem + (threadIdx.x >> 5) * asm_warp_bytes<TB, CPT>());
   uint4* st4 = reinterpret_cast<uint4*>(st);
   const int lane = threadIdx.x & 31;
-  const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t c = int64_t(blockIdx.x - (N.part ? 1 : 0)) * blockDim.x + threadIdx.x;
   const bool active = c < M.nc;
   int32_t e0 = 0, deg = 0;
   int64_t ci = 0, i = 0, ld = 0;
@@ -2297,7 +2337,11 @@ int ensure_material(fpsi_ctx* x) {
   return FPSI_OK;
 }
 
-int launch_residual(fpsi_ctx* x, double* resid_slot) {
+static dev::NormSink norm_sink(const fpsi_ctx* x, const NormOut& to) {
+  return dev::NormSink{to.rec ? x->d_part : nullptr, x->nblk_norm, x->d_err + 1, to};
+}
+
+int launch_residual(fpsi_ctx* x, double* rec) {
   const dev::MeshView M = view(x);
   const dev::Gas g = gas(x);
   cudaStream_t s = x->stream;
@@ -2409,7 +2453,7 @@ int launch_residual(fpsi_ctx* x, double* resid_slot) {
     dev::k_cell_residual<false><<<x->nblk_norm, dev::NORM_THREADS, 0, s>>>(
         M, x->d_q, x->d_F, g, x->P.urelax, x->P.dtmax, x->P.cflmax, x->H.vol_tot, nullptr, nullptr,
         x->d_src, x->d_dtau, x->d_part);
-  dev::k_norm_final<<<1, dev::NORM_THREADS, 0, s>>>(x->d_part, x->nblk_norm, x->d_err + 1, resid_slot);
+  if (rec) dev::k_norm_final<<<1, dev::NORM_THREADS, 0, s>>>(norm_sink(x, NormOut{rec, nullptr, nullptr}));
   prof_end(x);
   FPSI_CUDA_TRY(cudaGetLastError());
   return FPSI_OK;
@@ -2436,21 +2480,22 @@ static bool compact_blocks(const fpsi_ctx* x) {
 }
 
 template <class TB, class TX, bool CPT>
-static void launch_assemble_kernel(fpsi_ctx* x, const dev::MeshView& M, const dev::Gas& g) {
+static void launch_assemble_kernel(fpsi_ctx* x, const dev::MeshView& M, const dev::Gas& g, const NormOut& norms) {
   constexpr size_t smem = dev::asm_smem_bytes<TB, CPT>();
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(dev::k_assemble<TB, TX, CPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(smem));
-  dev::k_assemble<TB, TX, CPT><<<blocks_for(M.nc, dev::ASM_THREADS), dev::ASM_THREADS, smem, x->stream>>>(
+  const unsigned nb = blocks_for(M.nc, dev::ASM_THREADS) + (norms.rec ? 1 : 0);
+  dev::k_assemble<TB, TX, CPT><<<nb, dev::ASM_THREADS, smem, x->stream>>>(
       M, sweep_view(x), x->d_q, x->d_src, x->d_dtau, (const TB*)x->d_fjp, (const TB*)x->d_fjm,
       (const TB*)x->d_fjc, g, (TB*)x->d_luc, (TB*)x->d_bc, x->d_pv,
       x->P.solver == FPSI_SOLVER_LSGS ? nullptr : (TB*)x->d_aoff, x->keep_D ? (TB*)x->d_D : nullptr,
       (TX*)x->d_x, x->d_err, x->P.time_accurate ? 1.5 : 1.0,
-      x->any_fdbc ? (const TB*)x->d_bjac : nullptr);
+      x->any_fdbc ? (const TB*)x->d_bjac : nullptr, norm_sink(x, norms));
 }
 
 template <class TB, class TX>
-static int launch_assemble_t(fpsi_ctx* x) {
+static int launch_assemble_t(fpsi_ctx* x, const NormOut& norms) {
   const dev::MeshView M = view(x);
   const dev::Gas g = gas(x);
   cudaStream_t s = x->stream;
@@ -2482,25 +2527,25 @@ static int launch_assemble_t(fpsi_ctx* x) {
   }
   prof_begin(x, "assemble_lu");
   if (cpt)
-    launch_assemble_kernel<TB, TX, true>(x, M, g);
+    launch_assemble_kernel<TB, TX, true>(x, M, g, norms);
   else
-    launch_assemble_kernel<TB, TX, false>(x, M, g);
+    launch_assemble_kernel<TB, TX, false>(x, M, g, norms);
   prof_end(x);
   FPSI_CUDA_TRY(cudaGetLastError());
   return FPSI_OK;
 }
 
-int launch_assemble(fpsi_ctx* x) {
+int launch_assemble(fpsi_ctx* x, const NormOut& norms) {
   int rc;
   switch (x->P.precision) {
     case FPSI_PREC_FP64:
-      rc = launch_assemble_t<double, double>(x);
+      rc = launch_assemble_t<double, double>(x, norms);
       break;
     case FPSI_PREC_MIXED:
-      rc = launch_assemble_t<float, float>(x);
+      rc = launch_assemble_t<float, float>(x, norms);
       break;
     default:
-      rc = launch_assemble_t<float, double>(x);
+      rc = launch_assemble_t<float, double>(x, norms);
   }
   // FSGS starts its sweeps from zero (linearSolverFSGS.loci:1611), the
   // others from the block Jacobi solution the assembly left in x

@@ -8,9 +8,18 @@ struct fpsi_ctx;
 
 namespace fpsi {
 
+// where a residual's norms go: rec[NREC] (device) and, when given, the pinned
+// record host[NREC] -- of a run's step *seq (device, counted up) when seq is
+// given
+struct NormOut {
+  double* rec = nullptr;
+  double* host = nullptr;
+  int32_t* seq = nullptr;
+};
 // residual chain: boundary states, gradient+limiter, face flux, per-cell
-// gather (src, dtau), norms into resid_slot[8] (device)
-int launch_residual(fpsi_ctx* x, double* resid_slot);
+// gather (src, dtau), norms into rec[NREC] (device; null: left to the
+// launch_assemble that follows)
+int launch_residual(fpsi_ctx* x, double* rec);
 // the gradient-and-limiter records of the last residual's state (written
 // by the residual itself only for viscous runs)
 int launch_grad_records(fpsi_ctx* x);
@@ -19,8 +28,9 @@ int launch_grad_records(fpsi_ctx* x);
 // have changed since)
 int ensure_material(fpsi_ctx* x);
 // face Jacobians, diagonal blocks, LU, B and the starting iterate
-// (the starting iterate is the block Jacobi start D^-1 B)
-int launch_assemble(fpsi_ctx* x);
+// (the starting iterate is the block Jacobi start D^-1 B); with norms.rec one
+// block finishes the last residual's norms meanwhile
+int launch_assemble(fpsi_ctx* x, const NormOut& norms = {});
 // block Jacobi start x = D^-1 B on an assembled system
 int launch_jacobi_start(fpsi_ctx* x);
 // `sweeps` symmetric multi-colour Gauss-Seidel sweeps on the device iterate
