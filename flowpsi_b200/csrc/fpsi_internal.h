@@ -179,6 +179,7 @@ struct fpsi_ctx {
   // only for a longer run than any before)
   double* h_hist = nullptr;
   int64_t hist_cap = 0;
+  cudaGraphExec_t step_exec = nullptr;  // a run's step graph, rewritten by each run
   // state copy of fpsi_newton_step_ex, to undo a rejected update
   double* d_qsave = nullptr;   // [nc][5]
   int nblk_norm = 0;
