@@ -860,48 +860,75 @@ __global__ void k_loss_final(const double* __restrict__ part, int nblk, double* 
   }
 }
 
-// One layer of the backward pass, a CTA per rb cells (whole tiles of BT):
+// One layer of the backward pass, the tiles of BT cells split evenly over the
+// CTAs (at most as many as the device holds at once):
 //   dh  = Wo^T dy (TOP: the last layer, under the head), else the layer
 //         above's dh_in + its neighbour part: sum_{c in N} dagg_in[c] / deg(c)
 //         (the graph is symmetric)
 //   dz  = dh GELU'(z)
 //   part: the CTA's sums over its cells of dz x [h | agg] and dz (and, TOP,
-//         of dy x h_out and dy)
+//         of dy x h_out and dy), in nflush partials
 //   dh_out = dz Ws, dagg_out = dz Wn   (DENSE: every layer but the first)
-// The two products are FP32 FMAs: 16,384 per cell and hidden layer, which the
-// weights, dz and the layer's inputs feed from shared memory as 4 x 8 register
-// tiles, three 16 B loads per 32 FMAs.  Bound by the FMA pipe (ideal 0.2 ms
-// for 196,608 cells).  The layer's dz and its neighbour sums never reach
-// memory.  A loss-and-gradient call over 196,608 cells went from 5.68 to 1.14
-// ms (one thread per weight walking 256 cells before), over 1.57 M from 42.7
-// to 7.4; the neighbour gather of dagg_in is what keeps it from the FMA
-// rate.  Weight-gradient sums run over at most RB cells in FP32 in cell order
-// and across CTAs in FP64.
-constexpr int RB = 256;   // most cells per CTA and partial
+// The two products are FP32 FMAs: 16,384 per cell and hidden layer, fed from
+// shared memory as 4 x 8 and 8 x 4 register tiles in packed pairs (dz is
+// stored twice over, so that a pair of it needs no moves).  A CTA walks its
+// tiles: during a tile's weight gradient the next tile's dz is gathered
+// (neighbour ids, rows and sums a quarter of a tile apart) and its inputs
+// arrive by asynchronous copies, so that no load is waited for on its own.
+// dagg is divided by the degree where it is written, once per cell, not by
+// each reader.  196,608 cells, the three layers: 791 us with the tile's loads
+// in front of its products and 256 cells per CTA, 625 now; a
+// loss-and-gradient call 1.15 -> 0.97 ms (5.68 with one thread per weight),
+// over 1.57 M cells 7.4 -> 6.4, 24,576 0.28 -> 0.27.  The FMAs alone would
+// take 0.2 ms; what keeps it from them is the shared memory reads of dh_out's
+// product, which packed pairs made the bound (1.5 times its FMAs), and dz's
+// own arithmetic.  Weight-gradient sums run over at most RB cells in FP32 in
+// cell order and across partials in FP64.
+constexpr int RB = 256;   // most cells per partial
 constexpr int BT = 64;    // cells per tile
 constexpr int BTH = 256;  // threads per CTA
-constexpr int BZS = 68;   // floats per staged dz row: 16 B aligned, rows on different banks
+constexpr int BZS = 136;  // floats per staged dz row, each value twice: 16 B aligned, rows on different banks
 // floats of one CTA's partial: [64][2 fin] (Ws | Wn), b, then Wo, bo
 constexpr int back_part(int fin, bool top) { return W * 2 * fin + W + (top ? NOUT * W + NOUT : 0); }
 struct BackSmem {  // floats
-  int dz, a, w, dy, red, total;
+  int dz, a, w, dy, wo, off, red, total;
 };
 __host__ __device__ constexpr BackSmem back_smem(int fin, bool dense) {
   BackSmem s{};
   s.dz = 0;
   s.a = s.dz + BT * BZS;
-  s.w = s.a + BT * 2 * fin;
+  s.w = s.a + BT * 2 * fin;  // dense: two tiles of BF16 rows; else one of FP32
   s.dy = s.w + (dense ? W * 2 * fin : 0);
-  s.red = s.dy + BT * 8;
+  s.wo = s.dy + BT * 8;
+  s.off = s.wo + NOUT * W;
+  s.red = s.off + 2 * (BT + 4);
   s.total = s.red + 4 * (W + NOUT * W + 8);
   return s;
 }
 __device__ __forceinline__ void fma4(float4& a, float s, const float4& v) {
   a.x = fmaf(s, v.x, a.x), a.y = fmaf(s, v.y, a.y), a.z = fmaf(s, v.z, a.z), a.w = fmaf(s, v.w, a.w);
 }
+// two FMAs in one instruction, each rounded as fmaf; operands are register pairs
+__device__ __forceinline__ void fma2(float2& a, const float2& x, const float2& y) {
+  uint64_t& A = reinterpret_cast<uint64_t&>(a);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(A)
+      : "l"(reinterpret_cast<const uint64_t&>(x)), "l"(reinterpret_cast<const uint64_t&>(y)));
+}
+struct Pair2 {  // 16 B of shared memory as two register pairs
+  float2 lo, hi;
+};
+__device__ __forceinline__ Pair2 pair2(const float* p) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  return Pair2{make_float2(v.x, v.y), make_float2(v.z, v.w)};
+}
+__device__ __forceinline__ Pair2 pair2(const uint2& u) {  // four BF16
+  return Pair2{make_float2(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u)),
+               make_float2(__uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u))};
+}
 template <int FIN, bool TOP, bool DENSE, class TA>
 __global__ void __launch_bounds__(BTH, 2)
-k_back_layer(int64_t nc, int rb, const int32_t* __restrict__ off, const int32_t* __restrict__ nb,
+k_back_layer(int64_t nc, int nflush, const int32_t* __restrict__ off, const int32_t* __restrict__ nb,
              const float* __restrict__ z, const TA* __restrict__ h, const __nv_bfloat16* __restrict__ agg,
              const __nv_bfloat16* __restrict__ ws, const __nv_bfloat16* __restrict__ wn,
              const float* __restrict__ dh_in, const float* __restrict__ dagg_in,
@@ -913,203 +940,330 @@ k_back_layer(int64_t nc, int rb, const int32_t* __restrict__ off, const int32_t*
   static_assert(NC % 16 == 0 && (!DENSE || FIN == W), "tile shapes");
   extern __shared__ __align__(16) float bsm[];
   constexpr BackSmem S = back_smem(FIN, DENSE);
-  float *sdz = bsm + S.dz, *sa = bsm + S.a, *sw = bsm + S.w, *sdy = bsm + S.dy, *sred = bsm + S.red;
+  float *sdz = bsm + S.dz, *sa = bsm + S.a, *sw = bsm + S.w, *sdy = bsm + S.dy, *swo = bsm + S.wo, *sred = bsm + S.red;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (DENSE)
-    for (int i = t; i < W * NC; i += BTH) {
-      const int j = i / NC, k = i - NC * j;
-      sw[i] = __bfloat162float(k < FIN ? ws[j * FIN + k] : wn[j * FIN + k - FIN]);
+  if constexpr (DENSE) {
+    uint4 w8[W * NC / 8 / BTH];
+#pragma unroll
+    for (int u = 0; u < W * NC / 8 / BTH; ++u) {
+      const int i = t + u * BTH, j = i / (NC / 8), k = 8 * (i % (NC / 8));
+      w8[u] = __ldg(reinterpret_cast<const uint4*>(k < FIN ? ws + j * FIN + k : wn + j * FIN + k - FIN));
     }
+#pragma unroll
+    for (int u = 0; u < W * NC / 8 / BTH; ++u) {
+      const Pair2 a = pair2(make_uint2(w8[u].x, w8[u].y)), b = pair2(make_uint2(w8[u].z, w8[u].w));
+      float4* o = reinterpret_cast<float4*>(sw + 8 * (t + u * BTH));
+      o[0] = make_float4(a.lo.x, a.lo.y, a.hi.x, a.hi.y);
+      o[1] = make_float4(b.lo.x, b.lo.y, b.hi.x, b.hi.y);
+    }
+  }
+  if (TOP) {
+    for (int i = t; i < NOUT * W; i += BTH) swo[i] = __bfloat162float(wo[i]);
+  }
   const int jg = t >> 4, ig = t & 15;  // weight gradient: rows 4 jg.., columns of ig
-  float g[4][NI];
+  // NI == 8: columns 4 ig.. of both halves as pairs along the columns; else
+  // columns ig + 16 k, pairs along the rows
+  constexpr bool QUADS = NI == 8;
+  float2 g[QUADS ? 4 : 2][QUADS ? 4 : NI];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (auto& row : g)
 #pragma unroll
-    for (int k = 0; k < NI; ++k) g[r][k] = 0.f;
+    for (float2& v : row) v = make_float2(0.f, 0.f);
   const int bj = t & 63, bq = t >> 6;  // bias and head sums: feature bj, quarter of the tile's cells
   float gb = 0.f, gbo = 0.f, go[NOUT];
 #pragma unroll
   for (int k = 0; k < NOUT; ++k) go[k] = 0.f;
   double scale = 0.0;  // of dy, from the batch's size
   if (TOP) scale = loss_cnt[1] > 0 ? 2.0 / (5.0 * loss_cnt[1]) : 0.0;
-  const int64_t c0 = int64_t(blockIdx.x) * rb;
-  for (int64_t t0 = c0; t0 < min(c0 + rb, nc); t0 += BT) {
-    __syncthreads();  // the tile before is done with the staging
+  // the CTA's tiles, in nflush partials
+  const int64_t nt = (nc + BT - 1) / BT;
+  const int64_t tb = nt * blockIdx.x / gridDim.x, te = nt * (blockIdx.x + 1) / gridDim.x;
+  const int64_t c0 = tb * BT, c1 = min(te * BT, nc);
+  int nf = 0;  // partials written
+  auto flush_tile = [&]() { return tb + (te - tb) * (nf + 1) / nflush; };
+  int64_t flush_at = flush_tile();  // the tile that the next partial ends before
+  // ---- dz of the next tile, in registers: 16 threads a row, four features
+  // each (feature quad q), rows (t >> 4) + 16 r
+  const int q = t & 15;
+  float4 dn[BT / 16];       // TOP: z until its rows are staged
+  // the neighbour lists' ends of two tiles' cells: soff[parity][cell]
+  int32_t* soff = reinterpret_cast<int32_t*>(bsm + S.off);
+  auto ends = [&](int64_t tn) { return off[min(tn + t, nc)]; };  // threads 0..BT
+  int buf = 0;
+  if (t <= BT) soff[t] = ends(c0);
+  __syncthreads();
+  int32_t nid[4], ne = 0, ne1 = 0;
+  float4 nv[4], own, zz;
+  constexpr int NDY = (BT * NOUT + BTH - 1) / BTH;
+  float dyn[NDY];  // TOP: the next tile's dy
+  auto load_dy = [&](int64_t tn) {
+#pragma unroll
+    for (int u = 0; u < NDY; ++u) {
+      const int i = t + u * BTH;
+      dyn[u] = i < BT * NOUT && tn + i / NOUT < nc ? dy[tn * NOUT + i] : 0.f;
+    }
+  };
+  auto cell = [&](int64_t tn, int r) { return tn + (t >> 4) + 16 * r; };
+  // three steps apart, for the chain of loads: the first four neighbours' ids,
+  // their rows (an absent one adds zero), dz
+  auto ids = [&](int r, int b) {
+    const int32_t* e = soff + b * (BT + 4) + (t >> 4) + 16 * r;
+    ne = ne1 = 0;
+    if (!TOP) ne = e[0], ne1 = e[1];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) nid[u] = ne + u < ne1 ? nb[ne + u] : -1;
+  };
+  auto rows = [&](int64_t tn, int r) {
+    const int64_t cc = cell(tn, r);
+    own = zz = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (cc < c1) {
+      zz = *reinterpret_cast<const float4*>(z + cc * W + 4 * q);
+      if (!TOP) own = *reinterpret_cast<const float4*>(dh_in + cc * W + 4 * q);
+    }
+    if (!TOP) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        nv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (nid[u] >= 0) nv[u] = *reinterpret_cast<const float4*>(dagg_in + int64_t(nid[u]) * W + 4 * q);
+      }
+    }
+  };
+  int32_t le = 0, le1 = 0;  // the loaded row's neighbours past its first four
+  auto finish = [&](int r) {
+    float4 d = zz;
+    if (!TOP) {
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) sum.x += nv[u].x, sum.y += nv[u].y, sum.z += nv[u].z, sum.w += nv[u].w;
+      for (int32_t e = le + 4; e < le1; ++e) {
+        const float4 v = *reinterpret_cast<const float4*>(dagg_in + int64_t(nb[e]) * W + 4 * q);
+        sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+      }
+      d = own;
+      d.x += sum.x, d.y += sum.y, d.z += sum.z, d.w += sum.w;
+      d.x *= gelu_grad(zz.x), d.y *= gelu_grad(zz.y), d.z *= gelu_grad(zz.z), d.w *= gelu_grad(zz.w);
+    }
+    dn[r] = d;
+  };
+  // dense: a tile's inputs (BF16 already) into buffer b, rows past the end zero
+  __nv_bfloat16* sab = reinterpret_cast<__nv_bfloat16*>(sa);
+  auto inputs = [&](int64_t tn, int b) {
+    if constexpr (DENSE) {
+      if (tn >= c1) return;
+#pragma unroll
+      for (int u = 0; u < BT * NC / 8 / BTH; ++u) {
+        const int i = t + u * BTH, c = i / (NC / 8), k = i % (NC / 8);
+        const int64_t cc = tn + c;
+        const __nv_bfloat16* src =
+            k < FIN / 8 ? reinterpret_cast<const __nv_bfloat16*>(h) + (cc < nc ? cc : 0) * FIN + 8 * k
+                        : agg + (cc < nc ? cc : 0) * FIN + 8 * k - FIN;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         uint32_t(__cvta_generic_to_shared(sab + (b * BT + c) * NC + 8 * k))),
+                     "l"(src), "r"(cc < nc ? 16 : 0)
+                     : "memory");
+      }
+    }
+  };
+  inputs(c0, 0);
+  if (TOP) load_dy(c0);
+  ids(0, 0);
+#pragma unroll
+  for (int r = 0; r < BT / 16; ++r) {
+    rows(c0, r);
+    le = ne, le1 = ne1;
+    if (r + 1 < BT / 16) ids(r + 1, 0);
+    finish(r);
+  }
+  for (int64_t t0 = c0; t0 < c1; t0 += BT) {
+    if (DENSE) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // this tile's inputs are here, the tile before is done with the staging
+    if (DENSE) inputs(t0 + BT, buf ^ 1);
     if (TOP) {
-      for (int i = t; i < BT * NOUT; i += BTH) {
-        const int c = i / NOUT, k = i - NOUT * c;
-        sdy[8 * c + k] = t0 + c < nc ? float(double(dy[(t0 + c) * NOUT + k]) * scale) : 0.f;
+#pragma unroll
+      for (int u = 0; u < NDY; ++u) {
+        const int i = t + u * BTH, c = i / NOUT, k = i - NOUT * c;
+        if (i < BT * NOUT) sdy[8 * c + k] = float(double(dyn[u]) * scale);
       }
       __syncthreads();
     }
-    // ---- stage dz: 16 threads a row, four features each
+    int32_t next_end = 0;
+    if (t <= BT && t0 + BT < c1) next_end = ends(t0 + BT);
+    // ---- stage dz
 #pragma unroll
     for (int r = 0; r < BT / 16; ++r) {
-      const int c = (t >> 4) + 16 * r, q = t & 15;
-      const int64_t cc = t0 + c;
-      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cc < nc) {
-        if (TOP) {
+      const int c = (t >> 4) + 16 * r;
+      float4 d = dn[r];
+      if (TOP) {
+        const float4 zc = d;
+        d = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int k = 0; k < NOUT; ++k) {
-            const float v = sdy[8 * c + k];
-            const __nv_bfloat16* wr = wo + k * W + 4 * q;
-            fma4(d, v, make_float4(__bfloat162float(wr[0]), __bfloat162float(wr[1]), __bfloat162float(wr[2]),
-                                   __bfloat162float(wr[3])));
-          }
-        } else {
-          const int32_t e1 = off[cc + 1];
-          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int32_t e = off[cc]; e < e1; ++e) {
-            const int32_t o = nb[e];
-            const float deg = float(off[o + 1] - off[o]);
-            const float4 v = *reinterpret_cast<const float4*>(dagg_in + int64_t(o) * W + 4 * q);
-            sum.x += v.x / deg, sum.y += v.y / deg, sum.z += v.z / deg, sum.w += v.w / deg;
-          }
-          d = *reinterpret_cast<const float4*>(dh_in + cc * W + 4 * q);
-          d.x += sum.x, d.y += sum.y, d.z += sum.z, d.w += sum.w;
-        }
-        const float4 zz = *reinterpret_cast<const float4*>(z + cc * W + 4 * q);
-        d.x *= gelu_grad(zz.x), d.y *= gelu_grad(zz.y), d.z *= gelu_grad(zz.z), d.w *= gelu_grad(zz.w);
+        for (int k = 0; k < NOUT; ++k) fma4(d, sdy[8 * c + k], *reinterpret_cast<const float4*>(swo + k * W + 4 * q));
+        d.x *= gelu_grad(zc.x), d.y *= gelu_grad(zc.y), d.z *= gelu_grad(zc.z), d.w *= gelu_grad(zc.w);
       }
-      *reinterpret_cast<float4*>(sdz + c * BZS + 4 * q) = d;
+      float4* o = reinterpret_cast<float4*>(sdz + c * BZS + 8 * q);
+      o[0] = make_float4(d.x, d.x, d.y, d.y);
+      o[1] = make_float4(d.z, d.z, d.w, d.w);
     }
-    // ---- stage the layer's inputs as the forward GEMM used them
-    constexpr int CH = FIN / 8;  // 8-element chunks of one half row
-    for (int i = t; i < BT * 2 * CH; i += BTH) {
-      const int c = i / (2 * CH), q = i - 2 * CH * c;
-      const int64_t cc = t0 + c;
-      float v[8];
+    if (t <= BT) soff[(buf ^ 1) * (BT + 4) + t] = next_end;
+    __nv_bfloat16 hv[16];  // TOP: the quarter's hidden activations
+    if (TOP) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = 0.f;
-      if (cc < nc) {
-        if (q < CH) {
-          Chunk8<TA> ch;
-          ch.load(h + cc * FIN + 8 * q);
-          ch.get(v);
+      for (int c = 0; c < 16; ++c)
+        hv[c] = t0 + 16 * bq + c < nc ? hout[(t0 + 16 * bq + c) * W + bj] : __float2bfloat16_rn(0.f);
+    }
+    // ---- the first layer: stage its inputs as the forward GEMM used them
+    if constexpr (!DENSE) {
+      constexpr int CH = FIN / 8;  // 8-element chunks of one half row
+      constexpr int NCK = (BT * CH + BTH - 1) / BTH;
+      Chunk8<TA> ha[NCK];
+      Chunk8<__nv_bfloat16> ag[NCK];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = as_input<TA>(v[k]);
-        } else {
-          Chunk8<__nv_bfloat16> ch;
-          ch.load(agg + cc * FIN + 8 * (q - CH));
-          ch.get(v);
-        }
+      for (int u = 0; u < NCK; ++u) {
+        const int i = t + u * BTH;
+        const int64_t at = (t0 + i / CH < nc && i < BT * CH ? t0 * FIN + 8 * i : 0);
+        ha[u].load(h + at);
+        ag[u].load(agg + at);
       }
-      float4* o = reinterpret_cast<float4*>(sa + c * NC + 8 * q);
-      o[0] = make_float4(v[0], v[1], v[2], v[3]);
-      o[1] = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+      for (int u = 0; u < NCK; ++u) {
+        const int i = t + u * BTH, c = i / CH, k = i - CH * c;
+        if (c >= BT) continue;
+        const bool in = t0 + c < nc;
+        float v[8], w8[8];
+        ha[u].get(v);
+        ag[u].get(w8);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = in ? as_input<TA>(v[e]) : 0.f, w8[e] = in ? w8[e] : 0.f;
+        float4* o = reinterpret_cast<float4*>(sa + c * NC + 8 * k);
+        o[0] = make_float4(v[0], v[1], v[2], v[3]), o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        o = reinterpret_cast<float4*>(sa + c * NC + FIN + 8 * k);
+        o[0] = make_float4(w8[0], w8[1], w8[2], w8[3]), o[1] = make_float4(w8[4], w8[5], w8[6], w8[7]);
+      }
     }
     __syncthreads();
-    // ---- weight gradient: g[r][.] += dz[c][4 jg + r] a[c][.], cells in order
-    if constexpr (NI == 8) {
-#pragma unroll 4
-      for (int c = 0; c < BT; ++c) {
-        const float4 d = *reinterpret_cast<const float4*>(sdz + c * BZS + 4 * jg);
-        const float4 a0 = *reinterpret_cast<const float4*>(sa + c * NC + 4 * ig);
-        const float4 a1 = *reinterpret_cast<const float4*>(sa + c * NC + 64 + 4 * ig);
-        const float dv[4] = {d.x, d.y, d.z, d.w};
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) g[r][k] = fmaf(dv[r], av[k], g[r][k]);
-      }
-    } else {
-#pragma unroll 4
-      for (int c = 0; c < BT; ++c) {
-        const float4 d = *reinterpret_cast<const float4*>(sdz + c * BZS + 4 * jg);
-        const float dv[4] = {d.x, d.y, d.z, d.w};
-        float av[NI];
-#pragma unroll
-        for (int k = 0; k < NI; ++k) av[k] = sa[c * NC + ig + 16 * k];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int k = 0; k < NI; ++k) g[r][k] = fmaf(dv[r], av[k], g[r][k]);
-      }
-    }
-#pragma unroll 4
-    for (int c = 16 * bq; c < 16 * bq + 16; ++c) {
-      gb += sdz[c * BZS + bj];
+    for (int i = 0; i < 16; ++i) {
+      const int c = 16 * bq + i;
+      gb += sdz[c * BZS + 2 * bj];
       if (TOP) {
-        const float hv = t0 + c < nc ? __bfloat162float(hout[(t0 + c) * W + bj]) : 0.f;
+        const float v = __bfloat162float(hv[i]);
 #pragma unroll
-        for (int k = 0; k < NOUT; ++k) go[k] = fmaf(sdy[8 * c + k], hv, go[k]);
+        for (int k = 0; k < NOUT; ++k) go[k] = fmaf(sdy[8 * c + k], v, go[k]);
         if (bj < NOUT) gbo += sdy[8 * c + bj];
       }
     }
-    // ---- dh_out = dz Ws, dagg_out = dz Wn: warp w cells w + 8 k, lane four columns
+    // ---- dh_out = dz Ws, dagg_out = dz Wn / deg: a warp 16 cells and one of
+    // the two, its half warps alternate cells, a lane four columns
     if constexpr (DENSE) {
-      float4 acc[8];
+      const int half = warp & 1, cw = 16 * (warp >> 1) + (lane >> 4), cl = 4 * (lane & 15);
+      float2 acc[8][2];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = 0; k < 8; ++k) acc[k][0] = acc[k][1] = make_float2(0.f, 0.f);
 #pragma unroll 2
-      for (int j = 0; j < W; j += 4) {
-        float4 d[8], w4;
+      for (int j = 0; j < W; j += 2) {
+        const float* wj = sw + j * NC + W * half + cl;
+        const Pair2 w0 = pair2(wj), w1 = pair2(wj + NC);
+        Pair2 d[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) d[k] = *reinterpret_cast<const float4*>(sdz + (warp + 8 * k) * BZS + j);
-        w4 = *reinterpret_cast<const float4*>(sw + j * NC + 4 * lane);
+        for (int k = 0; k < 8; ++k) d[k] = pair2(sdz + (cw + 2 * k) * BZS + 2 * j);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].x, w4);
-        w4 = *reinterpret_cast<const float4*>(sw + (j + 1) * NC + 4 * lane);
+        for (int k = 0; k < 8; ++k) fma2(acc[k][0], d[k].lo, w0.lo), fma2(acc[k][1], d[k].lo, w0.hi);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].y, w4);
-        w4 = *reinterpret_cast<const float4*>(sw + (j + 2) * NC + 4 * lane);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].z, w4);
-        w4 = *reinterpret_cast<const float4*>(sw + (j + 3) * NC + 4 * lane);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) fma4(acc[k], d[k].w, w4);
+        for (int k = 0; k < 8; ++k) fma2(acc[k][0], d[k].hi, w1.lo), fma2(acc[k][1], d[k].hi, w1.hi);
       }
-      float* o = lane < 16 ? dh_out + 4 * lane : dagg_out + 4 * (lane - 16);
+      float* o = (half ? dagg_out : dh_out) + cl;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int64_t cc = t0 + warp + 8 * k;
-        if (cc < nc) *reinterpret_cast<float4*>(o + cc * W) = acc[k];
+        const int c = cw + 2 * k;
+        float4 v = make_float4(acc[k][0].x, acc[k][0].y, acc[k][1].x, acc[k][1].y);
+        if (half) {
+          const int32_t* e = soff + buf * (BT + 4) + c;
+          const float deg = float(e[1] - e[0]);
+          v.x /= deg, v.y /= deg, v.z /= deg, v.w /= deg;
+        }
+        if (t0 + c < nc) *reinterpret_cast<float4*>(o + (t0 + c) * W) = v;
       }
     }
-  }
-  // ---- the CTA's partials
-  float* o = part + int64_t(blockIdx.x) * back_part(FIN, TOP);
+    // ---- weight gradient: g[r][.] += dz[c][4 jg + r] a[c][.], cells in order,
+    // with the next tile's dz on its way
+    const int64_t tn = t0 + BT;
+    if (TOP && tn < c1) load_dy(tn);
+    if (tn < c1) ids(0, buf ^ 1);
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+    for (int r4 = 0; r4 < BT / 16; ++r4) {
+      if (tn < c1) {
+        rows(tn, r4);
+        le = ne, le1 = ne1;
+        if (r4 + 1 < BT / 16) ids(r4 + 1, buf ^ 1);
+      }
+#pragma unroll 4
+      for (int c = 16 * r4; c < 16 * r4 + 16; ++c) {
+        const Pair2 d0 = pair2(sdz + c * BZS + 8 * jg), d1 = pair2(sdz + c * BZS + 8 * jg + 4);
+        if constexpr (QUADS) {
+          const __nv_bfloat16* ar = sab + (buf * BT + c) * NC + 4 * ig;
+          const Pair2 a0 = pair2(*reinterpret_cast<const uint2*>(ar)), a1 = pair2(*reinterpret_cast<const uint2*>(ar + W));
+          const float2 dv[4] = {d0.lo, d0.hi, d1.lo, d1.hi};
 #pragma unroll
-    for (int k = 0; k < NI; ++k)
-      o[(4 * jg + r) * NC + (NI == 8 ? (k < 4 ? 4 * ig + k : 64 + 4 * ig + k - 4) : ig + 16 * k)] = g[r][k];
-  constexpr int RS = W + NOUT * W + 8;
-  __syncthreads();
-  sred[bq * RS + bj] = gb;
-  if (TOP) {
+          for (int r = 0; r < 4; ++r) {
+            fma2(g[r][0], dv[r], a0.lo);
+            fma2(g[r][1], dv[r], a0.hi);
+            fma2(g[r][2], dv[r], a1.lo);
+            fma2(g[r][3], dv[r], a1.hi);
+          }
+        } else {
+          const float2 p0 = make_float2(d0.lo.x, d0.hi.x), p1 = make_float2(d1.lo.x, d1.hi.x);
 #pragma unroll
-    for (int k = 0; k < NOUT; ++k) sred[bq * RS + W + k * W + bj] = go[k];
-    if (bj < NOUT) sred[bq * RS + W + NOUT * W + bj] = gbo;
-  }
-  __syncthreads();
-  for (int i = t; i < W + (TOP ? NOUT * W + NOUT : 0); i += BTH) {
-    float v = 0.f;
+          for (int k = 0; k < NI; ++k) {
+            const float av = sa[c * NC + ig + 16 * k];
+            fma2(g[0][k], p0, make_float2(av, av));
+            fma2(g[1][k], p1, make_float2(av, av));
+          }
+        }
+      }
+      if (tn < c1) finish(r4);
+    }
+    buf ^= 1;
+    if (t0 / BT + 1 < flush_at) continue;
+    // ---- a partial: the sums since the last one
+    float* o = part + (int64_t(blockIdx.x) * nflush + nf) * back_part(FIN, TOP);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v += sred[q * RS + i];
-    o[W * NC + i] = v;
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int k = 0; k < NI; ++k) {
+        const float2 v = QUADS ? g[r][k / 2] : g[r / 2][k];
+        o[(4 * jg + r) * NC + (QUADS ? (k < 4 ? 4 * ig + k : 64 + 4 * ig + k - 4) : ig + 16 * k)] =
+            (QUADS ? k : r) % 2 ? v.y : v.x;
+      }
+    constexpr int RS = W + NOUT * W + 8;
+    sred[bq * RS + bj] = gb;
+    if (TOP) {
+#pragma unroll
+      for (int k = 0; k < NOUT; ++k) sred[bq * RS + W + k * W + bj] = go[k];
+      if (bj < NOUT) sred[bq * RS + W + NOUT * W + bj] = gbo;
+    }
+    __syncthreads();
+    for (int i = t; i < W + (TOP ? NOUT * W + NOUT : 0); i += BTH) {
+      float v = 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v += sred[q * RS + i];
+      o[W * NC + i] = v;
+    }
+    ++nf;
+    flush_at = flush_tile();
+#pragma unroll
+    for (auto& row : g)
+#pragma unroll
+      for (float2& v : row) v = make_float2(0.f, 0.f);
+    gb = gbo = 0.f;
+#pragma unroll
+    for (int k = 0; k < NOUT; ++k) go[k] = 0.f;
   }
 }
 
-// Cells per CTA of k_back_layer on a device that holds `slots` of its CTAs at
-// once: whole tiles, at most RB, in the fewest rounds of CTAs times tiles
-// (a CTA's start and partial cost about a fifth of a tile).  1,296 cells
-// take 64 and spread over the device (a training step of 0.13 ms against
-// 0.24 with RB); 82,944 take 64 in five rounds, where RB would leave a
-// second round of 28 CTAs; large graphs take RB and write few partials.
-constexpr int64_t BACK_SMALL = 8;  // below RB only where that is at most this many rounds
-inline int back_cells(int64_t nc, int64_t slots) {
-  const int64_t nt = (nc + BT - 1) / BT;
-  int best = RB / BT;
-  double cost = 1e300;
-  for (int k = RB / BT; k >= 1; --k) {
-    const int64_t rounds = ((nt + k - 1) / k + slots - 1) / slots;
-    if (k < RB / BT && rounds > BACK_SMALL) break;
-    if (rounds * (k + 0.2) < cost) cost = rounds * (k + 0.2), best = k;
-  }
-  return best * BT;
+// Partials per CTA of k_back_layer when nt tiles are split evenly over ctas
+// (at most one each): none over more than RB cells.
+inline int back_partials(int64_t nt, int64_t ctas) {
+  return int(((nt + ctas - 1) / ctas * BT + RB - 1) / RB);
 }
 
 // the parameters' gradients from the CTAs' partials (np values each): a warp
@@ -1414,15 +1568,17 @@ int backward(fpsi_gnn* m, const Graph& G, const float* feat, const float* target
   float* dy = m->d_dz;  // [nc][5] fits in the [nc][64] buffer; read by the last layer only
   k_loss<<<nblk, GT, 0, s>>>(nc, m->d_y, target, seed, thr, mask, dy, m->d_lpart);
   k_loss_final<<<1, 256, 0, s>>>(m->d_lpart, nblk, loss_out);
-  const int rbc = back_cells(nc, 2 * m->nsm);
-  const unsigned rb = nb_(nc, rbc);
-  if (int64_t(rb) > m->part_cap) {
+  const int64_t nt = (nc + BT - 1) / BT;
+  const unsigned rb = unsigned(std::min<int64_t>(nt, 2 * m->nsm));
+  const int nf = back_partials(nt, rb);
+  const int64_t np_all = int64_t(rb) * nf;
+  if (np_all > m->part_cap) {
     FPSI_CUDA_TRY(cudaStreamSynchronize(s));
     if (m->d_part) cudaFree(m->d_part);
     m->part_cap = 0;
-    const int rc = galloc(&m->d_part, size_t(rb) * back_part(W, true));
+    const int rc = galloc(&m->d_part, size_t(np_all) * back_part(W, true));
     if (rc) return rc;
-    m->part_cap = rb;
+    m->part_cap = np_all;
   }
   // a layer reads the two parts of dh that the layer above wrote and writes
   // its own into the other pair of buffers
@@ -1434,18 +1590,18 @@ int backward(fpsi_gnn* m, const Graph& G, const float* feat, const float* target
     const __nv_bfloat16 *ws = m->d_wb + m->L.ws[l], *wn = m->d_wb + m->L.wn[l], *wo = m->d_wb + m->L.wo;
     if (top)
       k_back_layer<W, true, true, __nv_bfloat16><<<rb, BTH, smem, s>>>(
-          nc, rbc, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, nullptr, nullptr, dy, loss_out, wo,
+          nc, nf, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, nullptr, nullptr, dy, loss_out, wo,
           m->d_h[NLAYER], dh2, dagg2, m->d_part);
     else if (dense)
       k_back_layer<W, false, true, __nv_bfloat16><<<rb, BTH, smem, s>>>(
-          nc, rbc, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr,
+          nc, nf, G.off, G.nb, m->d_z[l], m->d_h[l], m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr,
           nullptr, dh2, dagg2, m->d_part);
     else
       k_back_layer<NIN, false, false, float><<<rb, BTH, smem, s>>>(
-          nc, rbc, G.off, G.nb, m->d_z[l], feat, m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr, nullptr,
+          nc, nf, G.off, G.nb, m->d_z[l], feat, m->d_agg[l], ws, wn, dh, dagg, nullptr, nullptr, nullptr, nullptr,
           nullptr, nullptr, m->d_part);
     const int np = back_part(fin, top);
-    k_back_reduce<<<nb_(np, 32), 32 * BRW, 0, s>>>(int(rb), np, fin, m->d_part, m->d_g,
+    k_back_reduce<<<nb_(np, 32), 32 * BRW, 0, s>>>(int(np_all), np, fin, m->d_part, m->d_g,
                                                   BackDst{m->L.ws[l], m->L.wn[l], m->L.b[l], m->L.wo, m->L.bo});
     std::swap(dh, dh2);
     std::swap(dagg, dagg2);
