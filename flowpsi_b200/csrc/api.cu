@@ -760,10 +760,8 @@ int fpsi_residual(fpsi_ctx* x, double* src, fpsi_resid* norms) {
   int rc;
   x->have_sa = x->have_sa_dq = false;
   if (fpsi::sa_active(x) && (rc = fpsi::sa_launch_tmu(x))) return rc;
-  rc = fpsi::launch_residual(x, x->d_resid);
+  rc = fpsi::launch_residual(x, {x->d_resid, x->h_resid, nullptr});
   if (rc) return rc;
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid, x->d_resid, fpsi::NREC * sizeof(double),
-                                cudaMemcpyDeviceToHost, x->stream));
   if ((rc = src ? rows_down(x, 5, nullptr, x->d_src, 8, src) : sync(x))) return rc;
   if (norms) fill_norms(x, x->h_resid, norms);
   x->have_resid = true;
@@ -982,10 +980,8 @@ int fpsi_linear_sweeps(fpsi_ctx* x, int32_t nsweeps) {
 int fpsi_linear_residual(fpsi_ctx* x, double* norm_b, double* norm_r) {
   if (!x) return FPSI_E_INVALID;
   if (!x->have_asm || !x->d_D) return FPSI_E_STATE;
-  int rc = fpsi::launch_linres(x, x->d_resid + 16);
+  int rc = fpsi::launch_linres(x, x->d_resid + 16, x->h_resid + 16);
   if (rc) return rc;
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid + 16, x->d_resid + 16, 2 * sizeof(double),
-                                cudaMemcpyDeviceToHost, x->stream));
   if ((rc = sync(x))) return rc;
   if (norm_b) *norm_b = x->h_resid[16];
   if (norm_r) *norm_r = x->h_resid[17];
@@ -1011,7 +1007,7 @@ int fpsi_newton_step(fpsi_ctx* x, fpsi_stepinfo* info) {
   int rc;
   const bool sa = fpsi::sa_active(x);
   if (sa && (rc = fpsi::sa_launch_tmu(x))) return rc;
-  if ((rc = fpsi::launch_residual(x, nullptr))) return rc;
+  if ((rc = fpsi::launch_residual(x))) return rc;
   if (sa && ((rc = fpsi::sa_launch_residual(x)) || (rc = fpsi::sa_launch_solve(x)))) return rc;
   if ((rc = fpsi::launch_assemble(x, {x->d_resid, x->h_resid, nullptr}))) return rc;
   if (is_lsgs(x)) {
@@ -1060,9 +1056,7 @@ int ex_sweeps(fpsi_ctx* x, const fpsi_step_opts& o, fpsi_lsinfo* info) {
   const int every = std::max(1, o.check_every);
   int done = 0;
   for (bool first = true;; first = false) {
-    if ((rc = fpsi::launch_linres(x, x->d_resid + 16))) return rc;
-    FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid + 16, x->d_resid + 16, 2 * sizeof(double),
-                                  cudaMemcpyDeviceToHost, x->stream));
+    if ((rc = fpsi::launch_linres(x, x->d_resid + 16, x->h_resid + 16))) return rc;
     if ((rc = sync(x))) return rc;
     const double nb = x->h_resid[16], nr = x->h_resid[17];
     if (first) info->resid0 = nr;
@@ -1078,10 +1072,8 @@ int ex_sweeps(fpsi_ctx* x, const fpsi_step_opts& o, fpsi_lsinfo* info) {
 
 // residual of the current state into d_resid and h_resid
 int ex_residual(fpsi_ctx* x) {
-  int rc = fpsi::launch_residual(x, x->d_resid);
+  int rc = fpsi::launch_residual(x, {x->d_resid, x->h_resid, nullptr});
   if (rc) return rc;
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->h_resid, x->d_resid, fpsi::NREC * sizeof(double),
-                                cudaMemcpyDeviceToHost, x->stream));
   if ((rc = sync(x))) return rc;
   x->have_resid = true;
   x->have_asm = x->have_dq = x->x_preset = false;
@@ -1205,7 +1197,7 @@ int fpsi_newton_step_ex(fpsi_ctx* x, fpsi_gnn* model, const fpsi_step_opts* opts
 static int launch_step(fpsi_ctx* x, bool sa) {
   int rc = FPSI_OK;
   if (sa) rc = fpsi::sa_launch_tmu(x);
-  if (!rc) rc = fpsi::launch_residual(x, nullptr);
+  if (!rc) rc = fpsi::launch_residual(x);
   if (!rc && sa) rc = fpsi::sa_launch_residual(x);
   if (!rc && sa) rc = fpsi::sa_launch_solve(x);
   if (!rc) rc = fpsi::launch_assemble(x, {x->d_resid, x->h_hist, x->d_err + 2});

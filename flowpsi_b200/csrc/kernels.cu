@@ -1131,6 +1131,7 @@ __device__ __forceinline__ void norm_final(const NormSink& N, double (*sh)[NORM_
 #pragma unroll 1
   for (int v = t; v < NORM_THREADS; v += T) {
     double a[8] = {0, 0, 0, 0, -1, 0, -1, 0};
+#pragma unroll 2
     for (int i = v; i < N.nblk; i += NORM_THREADS) {
       const double* p = N.part + 8 * int64_t(i);
       a[0] += p[0], a[1] += p[1], a[2] += p[2];
@@ -2073,10 +2074,14 @@ k_linres_slots(const ColInfo* __restrict__ col, const int32_t* __restrict__ cell
   }
 }
 
-__global__ void k_sum2(const double* __restrict__ part, int nblk, double* __restrict__ out) {
+// out and, straight to the host, the pinned host[2] (a copy behind the kernel
+// cost a check of a solve to a tolerance 17 of its 215 us, 663,552 cells)
+__global__ void k_sum2(const double* __restrict__ part, int nblk, double* __restrict__ out,
+                       volatile double* host) {
   __shared__ double sh[2][NORM_THREADS];
   const int t = threadIdx.x;
   double a = 0, b = 0;
+#pragma unroll 8
   for (int i = t; i < nblk; i += NORM_THREADS) a += part[2 * i], b += part[2 * i + 1];
   sh[0][t] = a, sh[1][t] = b;
   __syncthreads();
@@ -2084,7 +2089,7 @@ __global__ void k_sum2(const double* __restrict__ part, int nblk, double* __rest
     if (t < st) sh[0][t] += sh[0][t + st], sh[1][t] += sh[1][t + st];
     __syncthreads();
   }
-  if (t == 0) out[0] = sqrt(sh[0][0]), out[1] = sqrt(sh[1][0]);
+  if (t == 0) host[0] = out[0] = sqrt(sh[0][0]), host[1] = out[1] = sqrt(sh[1][0]);
 }
 
 // ---------------------------------------------------------------------------
@@ -2341,7 +2346,7 @@ static dev::NormSink norm_sink(const fpsi_ctx* x, const NormOut& to) {
   return dev::NormSink{to.rec ? x->d_part : nullptr, x->nblk_norm, x->d_err + 1, to};
 }
 
-int launch_residual(fpsi_ctx* x, double* rec) {
+int launch_residual(fpsi_ctx* x, const NormOut& norms) {
   const dev::MeshView M = view(x);
   const dev::Gas g = gas(x);
   cudaStream_t s = x->stream;
@@ -2453,7 +2458,7 @@ int launch_residual(fpsi_ctx* x, double* rec) {
     dev::k_cell_residual<false><<<x->nblk_norm, dev::NORM_THREADS, 0, s>>>(
         M, x->d_q, x->d_F, g, x->P.urelax, x->P.dtmax, x->P.cflmax, x->H.vol_tot, nullptr, nullptr,
         x->d_src, x->d_dtau, x->d_part);
-  if (rec) dev::k_norm_final<<<1, dev::NORM_THREADS, 0, s>>>(norm_sink(x, NormOut{rec, nullptr, nullptr}));
+  if (norms.rec) dev::k_norm_final<<<1, dev::NORM_THREADS, 0, s>>>(norm_sink(x, norms));
   prof_end(x);
   FPSI_CUDA_TRY(cudaGetLastError());
   return FPSI_OK;
@@ -2652,7 +2657,7 @@ int ensure_explicit_blocks(fpsi_ctx* x) {
 }
 
 template <class TB, class TX>
-static int launch_linres_t(fpsi_ctx* x, double* out2) {
+static int launch_linres_t(fpsi_ctx* x, double* out2, double* host2) {
   int64_t nblk = x->nblk_norm;
   if (x->P.solver == FPSI_SOLVER_LSGS) {
     // the line solver's system has explicit blocks
@@ -2667,19 +2672,19 @@ static int launch_linres_t(fpsi_ctx* x, double* out2) {
                                                         (const TB*)x->d_aoff, (const TB*)x->d_bc, (const TB*)x->d_D,
                                                         (const TX*)x->d_x, x->d_part);
   }
-  dev::k_sum2<<<1, dev::NORM_THREADS, 0, x->stream>>>(x->d_part, int(nblk), out2);
+  dev::k_sum2<<<1, dev::NORM_THREADS, 0, x->stream>>>(x->d_part, int(nblk), out2, host2);
   FPSI_CUDA_TRY(cudaGetLastError());
   return FPSI_OK;
 }
 
-int launch_linres(fpsi_ctx* x, double* out2) {
+int launch_linres(fpsi_ctx* x, double* out2, double* host2) {
   switch (x->P.precision) {
     case FPSI_PREC_FP64:
-      return launch_linres_t<double, double>(x, out2);
+      return launch_linres_t<double, double>(x, out2, host2);
     case FPSI_PREC_MIXED:
-      return launch_linres_t<float, float>(x, out2);
+      return launch_linres_t<float, float>(x, out2, host2);
     default:
-      return launch_linres_t<float, double>(x, out2);
+      return launch_linres_t<float, double>(x, out2, host2);
   }
 }
 

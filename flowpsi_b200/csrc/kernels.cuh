@@ -17,9 +17,9 @@ struct NormOut {
   int32_t* seq = nullptr;
 };
 // residual chain: boundary states, gradient+limiter, face flux, per-cell
-// gather (src, dtau), norms into rec[NREC] (device; null: left to the
+// gather (src, dtau) and, with norms.rec, the norms (else left to the
 // launch_assemble that follows)
-int launch_residual(fpsi_ctx* x, double* rec);
+int launch_residual(fpsi_ctx* x, const NormOut& norms = {});
 // the gradient-and-limiter records of the last residual's state (written
 // by the residual itself only for viscous runs)
 int launch_grad_records(fpsi_ctx* x);
@@ -35,8 +35,8 @@ int launch_assemble(fpsi_ctx* x, const NormOut& norms = {});
 int launch_jacobi_start(fpsi_ctx* x);
 // `sweeps` symmetric multi-colour Gauss-Seidel sweeps on the device iterate
 int launch_sgs(fpsi_ctx* x, int sweeps);
-// out2[0] = ||B||, out2[1] = ||B - A x|| (device)
-int launch_linres(fpsi_ctx* x, double* out2);
+// out2[0] = ||B||, out2[1] = ||B - A x|| (device), and the pinned host2 too
+int launch_linres(fpsi_ctx* x, double* out2, double* host2);
 // fills fjp/fjm from the compact face records of the assembled system (a
 // no-op when they already hold it)
 int ensure_explicit_blocks(fpsi_ctx* x);
