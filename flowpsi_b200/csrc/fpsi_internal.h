@@ -164,9 +164,10 @@ struct fpsi_ctx {
   double* d_src = nullptr;     // [nc][5]
   double* d_dtau = nullptr;    // [nc]
   double* d_tmu = nullptr;     // [nc] eddy viscosity (flowRegime turbulent)
-  double* d_muk = nullptr;     // [nc][2] Sutherland viscosity and conductivity of the last
-                               // residual's state (viscous runs; made on first use)
-  double muk_with[6] = {0, 0, 0, 0, 0, 0};  // the Sutherland constants of d_muk
+  double* d_muk = nullptr;     // [nc][2] Sutherland viscosity and conductivity of each cell
+                               // (viscous runs; made on first use)
+  bool muk_valid = false;      // d_muk holds them for the last residual's state ...
+  double muk_with[6] = {0, 0, 0, 0, 0, 0};  // ... with these constants
   double* d_part = nullptr;    // per-block partial norms
   double* d_resid = nullptr;   // 16 doubles: final norms
   double* h_resid = nullptr;   // pinned mirror

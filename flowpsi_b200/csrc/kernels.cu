@@ -2316,23 +2316,27 @@ void launch_grad(fpsi_ctx* x, const dev::MeshView& M, cudaStream_t s) {
   }
 }
 
+// d_muk holds the current state's laws with the constants in force: a kernel
+// that fills it (material_cell) has been launched
+static void note_material(fpsi_ctx* x) {
+  if (!x->P.viscous || !x->d_muk) return;  // visc() gave it no array to fill
+  const double m[6] = {x->P.mu_a1, x->P.mu_a2, x->P.mu_a3, x->P.k_a1, x->P.k_a2, x->P.k_a3};
+  for (int i = 0; i < 6; ++i) x->muk_with[i] = m[i];
+  x->muk_valid = true;
+}
+
 int launch_grad_records(fpsi_ctx* x) {
   const dev::MeshView M = view(x);
   launch_grad<true>(x, M, x->stream);
   FPSI_CUDA_TRY(cudaGetLastError());
+  note_material(x);
   x->grad_valid = true;
   return FPSI_OK;
 }
 
-// the Sutherland constants d_muk was computed with
-static void note_material(fpsi_ctx* x) {
-  const double m[6] = {x->P.mu_a1, x->P.mu_a2, x->P.mu_a3, x->P.k_a1, x->P.k_a2, x->P.k_a3};
-  for (int i = 0; i < 6; ++i) x->muk_with[i] = m[i];
-}
-
 int ensure_material(fpsi_ctx* x) {
   const double m[6] = {x->P.mu_a1, x->P.mu_a2, x->P.mu_a3, x->P.k_a1, x->P.k_a2, x->P.k_a3};
-  bool same = x->d_muk != nullptr;
+  bool same = x->muk_valid;
   for (int i = 0; i < 6; ++i) same = same && x->muk_with[i] == m[i];
   if (same) return FPSI_OK;
   if (!x->d_muk) FPSI_CUDA_TRY(cudaMalloc(&x->d_muk, size_t(x->H.nc) * 2 * sizeof(double)));
@@ -2372,18 +2376,19 @@ int launch_residual(fpsi_ctx* x, const NormOut& norms) {
       x->ageom_factor = x->P.lds_nonsym_factor;
     }
   }
-  if (x->P.viscous) {
-    if (!x->d_muk) FPSI_CUDA_TRY(cudaMalloc(&x->d_muk, size_t(M.nc) * 2 * sizeof(double)));
-    note_material(x);
-  }
+  // the laws kept are an older state's from here on, until a kernel fills them
+  x->muk_valid = false;
+  if (x->P.viscous && !x->d_muk) FPSI_CUDA_TRY(cudaMalloc(&x->d_muk, size_t(M.nc) * 2 * sizeof(double)));
   prof_begin(x, "grad_limiter");
   // the gradient records are written every residual only where the viscous
   // terms, the SA model and the KEC flux read them
   x->grad_valid = x->P.viscous != 0 || kec;
-  if (x->grad_valid)
+  if (x->grad_valid) {
     launch_grad<true>(x, M, s);
-  else
+    note_material(x);
+  } else {
     launch_grad<false>(x, M, s);
+  }
   if (kec)
     dev::k_alpha_diss<<<blocks_for(M.nc, dev::AD_THREADS), dev::AD_THREADS, 0, s>>>(
         M, x->d_q, x->d_qb, x->d_grad, g, lds(x), x->d_adiss);

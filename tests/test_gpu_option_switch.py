@@ -1,0 +1,69 @@
+"""Options that change between a residual and what is built from it: the
+assembly uses the last residual's state with the options in force, as a new
+context that was given those options from the start.  GPU only."""
+import numpy as np
+import pytest
+
+from flowpsi_b200 import FlowPsi, cases
+from flowpsi_b200._native import FLUX
+from tests.helpers import block_rel
+
+pytestmark = pytest.mark.gpu
+
+# FP32 blocks: both sides evaluate the same formulas in FP64 and round once
+# (the bars of test_gpu_viscous.py)
+TOL = {"ref": 1e-6, "fp64": 1e-11}
+
+
+def _case(flux, prec):
+    c = cases.boundary_layer_block(6, 8, 4, dy0=1e-3, growth=1.3, viscous=1, precision=prec, solver="sgs")
+    c.params.flux = FLUX[flux]
+    return c
+
+
+def _states(g, c):
+    T, p, u = c.initial_state(g.geometry()["cellcenter"])
+    r = np.random.default_rng(5)
+    a = (T * (1.0 + 0.1 * r.random(T.size)), p, u)
+    b = (2.5 * T * (1.0 + 0.1 * r.random(T.size)), p, u * (1.0 + 0.1 * r.random(u.shape)))
+    return a, b
+
+
+def _blocks(g):
+    g.assemble()
+    return g.blocks()
+
+
+def _compare(got, want, prec):
+    for k in ("fjp", "fjm"):
+        inner = np.abs(want[k]).reshape(len(want[k]), -1).max(1) > 0
+        assert block_rel(got[k][inner], want[k][inner]) < TOL[prec], k
+
+
+@pytest.mark.parametrize("prec", ["ref", "fp64"])
+def test_viscosity_follows_the_state_of_an_inviscid_residual(need_gpu, prec):
+    """viscous on state A, inviscid on state B, viscous again: the KEC flux
+    keeps the gradient records of B, the viscosities have to be B's too"""
+    c = _case("kec", prec)
+    g = FlowPsi(c.mesh, c.params)
+    A, B = _states(g, c)
+    p = g.params
+    g.set_state(*A)
+    g.residual()
+    p.viscous = 0
+    g.set_params(p)
+    g.set_state(*B)
+    g.residual()
+    p.viscous = 1
+    g.set_params(p)
+    got = _blocks(g)
+    # the time step is the inviscid residual's: the new context switches as well
+    d = _case("kec", prec)
+    d.params.viscous = 0
+    f = FlowPsi(d.mesh, d.params)
+    f.set_state(*B)
+    f.residual()
+    d.params.viscous = 1
+    f.set_params(d.params)
+    _compare(got, _blocks(f), prec)
+    f.close(), g.close()

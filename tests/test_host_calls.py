@@ -1,0 +1,46 @@
+"""What the library's host code asks of the CUDA runtime, with the runtime of
+tests/fake_cudart.c in front of it: no GPU, no kernel runs."""
+from tests.fake_runtime import run
+
+VISCOUS = """
+c = cases.boundary_layer_block(4, 6, 3, dy0=1e-3, growth=1.3, viscous=1, precision="ref", solver="sgs")
+c.params.flux = FLUX
+g = FlowPsi(c.mesh, c.params)
+st = c.initial_state(g.geometry()["cellcenter"])
+p = g.params
+def viscous(v):
+    p.viscous = v
+    g.set_params(p)
+def since(n, pattern):
+    return [c.name for c in calls[n:] if c.what == "launch" and pattern in c.name]
+"""
+
+
+def test_viscosities_of_an_older_state_are_made_again():
+    """the cells' viscosities are kept per state: an inviscid residual (here
+    with the flux that keeps its gradient records) leaves them behind"""
+    run(VISCOUS.replace("FLUX", "3") + """
+g.set_state(*st); g.residual()
+n = len(calls); g.assemble()
+assert not since(n, "k_material")        # the residual's own
+viscous(0); g.residual()
+viscous(1); n = len(calls); g.assemble()
+assert len(since(n, "k_material")) == 1  # not the first residual's
+n = len(calls); g.assemble()
+assert not since(n, "k_material")
+p.mu_a1 *= 1.5; g.set_params(p); n = len(calls); g.assemble()
+assert len(since(n, "k_material")) == 1  # other constants
+""")
+
+
+def test_viscosities_follow_the_constants_of_the_gradient_records():
+    """records made on request fill the viscosities with the constants then in
+    force; going back to the earlier constants is a change too"""
+    run(VISCOUS.replace("FLUX", "1") + """
+g.set_state(*st); g.residual()
+viscous(0); g.residual()
+viscous(1); a = p.mu_a1; p.mu_a1 = 1.5 * a; g.set_params(p)
+g.reconstruction()
+p.mu_a1 = a; g.set_params(p); n = len(calls); g.assemble()
+assert len(since(n, "k_material")) == 1
+""")
