@@ -2513,7 +2513,8 @@ static int launch_assemble_t(fpsi_ctx* x, const NormOut& norms) {
   TB* fjm = (TB*)x->d_fjm;
   const bool cpt = compact_blocks(x);
   if (x->P.viscous) {
-    const int rc = ensure_material(x);
+    int rc = x->grad_valid ? FPSI_OK : launch_grad_records(x);
+    if (!rc) rc = ensure_material(x);
     if (rc) return rc;
   }
   x->asm_compact = cpt;

@@ -20,8 +20,8 @@ struct NormOut {
 // gather (src, dtau) and, with norms.rec, the norms (else left to the
 // launch_assemble that follows)
 int launch_residual(fpsi_ctx* x, const NormOut& norms = {});
-// the gradient-and-limiter records of the last residual's state (written
-// by the residual itself only for viscous runs)
+// the gradient-and-limiter records of the last residual's state, where the
+// residual did not write them (!grad_valid: it was inviscid)
 int launch_grad_records(fpsi_ctx* x);
 // the cells' viscosity and conductivity, for the last residual's state and the
 // options in force (the residual of a viscous run leaves them; options may

@@ -453,7 +453,8 @@ int sa_launch_tmu(fpsi_ctx* x) {
 }
 
 int sa_launch_residual(fpsi_ctx* x) {
-  const int rc = ensure_material(x);
+  int rc = x->grad_valid ? FPSI_OK : launch_grad_records(x);
+  if (!rc) rc = ensure_material(x);
   if (rc) return rc;
   const sa::Geo G = geo(x);
   const sa::Gas g = sgas(x);

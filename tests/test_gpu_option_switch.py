@@ -67,3 +67,28 @@ def test_viscosity_follows_the_state_of_an_inviscid_residual(need_gpu, prec):
     f.set_params(d.params)
     _compare(got, _blocks(f), prec)
     f.close(), g.close()
+
+
+@pytest.mark.parametrize("prec", ["ref", "fp64"])
+def test_viscous_blocks_after_an_inviscid_residual(need_gpu, prec):
+    """viscous on state A, inviscid (Roe: no gradient records) on state B,
+    viscous again: the face Jacobians are those of a viscous context on B"""
+    c = _case("roe", prec)
+    g = FlowPsi(c.mesh, c.params)
+    A, B = _states(g, c)
+    p = g.params
+    g.set_state(*A)
+    g.residual()
+    p.viscous = 0
+    g.set_params(p)
+    g.set_state(*B)
+    g.residual()
+    p.viscous = 1
+    g.set_params(p)
+    got = _blocks(g)
+    d = _case("roe", prec)
+    f = FlowPsi(d.mesh, d.params)
+    f.set_state(*B)
+    f.residual()
+    _compare(got, _blocks(f), prec)
+    f.close(), g.close()

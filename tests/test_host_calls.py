@@ -44,3 +44,22 @@ g.reconstruction()
 p.mu_a1 = a; g.set_params(p); n = len(calls); g.assemble()
 assert len(since(n, "k_material")) == 1
 """)
+
+
+def test_gradient_records_of_an_inviscid_residual_are_made_for_viscous_blocks():
+    """an inviscid Roe residual writes no gradient records; the viscous face
+    Jacobians and the SA system read them"""
+    run(VISCOUS.replace("FLUX", "1") + """
+g.set_state(*st); g.residual()
+n = len(calls); g.assemble()
+assert not since(n, "k_grad")            # the residual's own
+viscous(0); g.residual()
+viscous(1); n = len(calls); g.assemble()
+k = [c for c in since(n, "k_grad") + since(n, "k_face_jacobian")]
+assert len(k) == 2 and "k_grad" in k[0] and "ILb1E" in k[0], k
+n = len(calls); g.assemble()
+assert not since(n, "k_grad")
+viscous(0); g.residual()
+p.viscous = 2; p.turbulence = 1; g.set_params(p); n = len(calls); g.sa_residual()
+assert len(since(n, "k_grad")) == 1
+""")
