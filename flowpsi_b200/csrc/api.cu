@@ -103,6 +103,7 @@ int alloc_system(fpsi_ctx* x) {
     return rc;
   x->alloc_prec = x->P.precision;
   x->have_asm = x->have_dq = false;
+  x->jac_fresh = 0;  // the flux kernel's face records went with the old arrays
   return FPSI_OK;
 }
 

@@ -63,3 +63,28 @@ viscous(0); g.residual()
 p.viscous = 2; p.turbulence = 1; g.set_params(p); n = len(calls); g.sa_residual()
 assert len(since(n, "k_grad")) == 1
 """)
+
+
+def test_face_records_are_made_again_in_new_system_arrays():
+    """the flux kernel leaves the compact face Jacobians of an inviscid
+    residual; keeping the diagonal blocks or another precision allocates the
+    system anew"""
+    run("""
+c = cases.farfield_cube(4, precision="ref")
+g = FlowPsi(c.mesh, c.params)
+g.set_state(*c.initial_state(g.geometry()["cellcenter"]))
+def made(change):
+    g.residual()
+    change()
+    n = len(calls); g.assemble()
+    return len([c for c in calls[n:] if c.what == "launch" and "k_face_jacobian_c" in c.name])
+assert made(lambda: None) == 0
+assert made(lambda: g.keep_blocks(False)) == 1
+assert made(lambda: None) == 0
+assert made(lambda: g.keep_blocks(True)) == 1
+def mixed():
+    p = g.params
+    p.precision = 2  # FP32 blocks as before
+    g.set_params(p)
+assert made(mixed) == 1
+""")
