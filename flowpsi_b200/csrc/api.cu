@@ -540,6 +540,8 @@ int fpsi_set_params(fpsi_ctx* x, const fpsi_params* p) {
   if (!x) return FPSI_E_INVALID;
   int rc = check_params(p);
   if (rc) return rc;
+  // the face records the last residual left are of its gas
+  if (p->gamma != x->P.gamma || p->Rtilde != x->P.Rtilde || p->Pambient != x->P.Pambient) x->jac_fresh = 0;
   x->P = *p;
   x->have_asm = x->have_dq = x->have_xprev = false;
   x->have_levels = false;

@@ -92,3 +92,30 @@ def test_viscous_blocks_after_an_inviscid_residual(need_gpu, prec):
     f.residual()
     _compare(got, _blocks(f), prec)
     f.close(), g.close()
+
+
+@pytest.mark.parametrize("prec", ["ref", "fp64"])
+def test_face_records_follow_the_gas(need_gpu, prec):
+    """gamma changed between an inviscid residual and the assembly: the face
+    Jacobians are those of the new gas (the face states' pressures,
+    temperatures and velocities, first order here, do not depend on it)"""
+    c = cases.farfield_cube(6, precision=prec, limiter="zero")
+    g = FlowPsi(c.mesh, c.params)
+    st = c.initial_state(g.geometry()["cellcenter"])
+    g.set_state(*st)
+    g.residual()
+    p = g.params
+    p.gamma = 1.3
+    g.set_params(p)
+    got = _blocks(g)
+    d = cases.farfield_cube(6, precision=prec, limiter="zero")
+    d.params.gamma = 1.3
+    f = FlowPsi(d.mesh, d.params)
+    f.set_state(*st)
+    f.residual()
+    want = _blocks(f)
+    # interior faces: a boundary state may depend on gamma
+    inner = d.mesh.arrays().cr >= 0
+    for k in ("fjp", "fjm"):
+        assert block_rel(got[k][inner], want[k][inner]) < TOL[prec], k
+    f.close(), g.close()
