@@ -897,9 +897,12 @@ int fpsi_get_blocks(fpsi_ctx* x, void* D, void* fjp, void* fjm, void* B) {
   return FPSI_OK;
 }
 
-// the iterate: colour order, or line order (whose padding rows stay as they are)
+// the iterate: colour order, or line order, whose padding rows are zero (they
+// enter the line solver's residual; a solve that diverged leaves NaN there)
 static int upload_x(fpsi_ctx* x, const double* x0) {
-  return is_lsgs(x) ? rows_up(x, 5, x->d_lt, x0, x->d_lx, x->x_bytes) : rows_up(x, 5, x->d_ci, x0, x->d_x, x->x_bytes);
+  if (!is_lsgs(x)) return rows_up(x, 5, x->d_ci, x0, x->d_x, x->x_bytes);
+  FPSI_CUDA_TRY(cudaMemsetAsync(x->d_lx, 0, size_t(x->LY.nrows) * 32 * 5 * x->x_bytes, x->stream));
+  return rows_up(x, 5, x->d_lt, x0, x->d_lx, x->x_bytes);
 }
 
 static int download_x(fpsi_ctx* x, double* dq) {

@@ -119,3 +119,37 @@ def test_face_records_follow_the_gas(need_gpu, prec):
     for k in ("fjp", "fjm"):
         assert block_rel(got[k][inner], want[k][inner]) < TOL[prec], k
     f.close(), g.close()
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_line_solve_from_a_given_start_after_a_diverged_one(need_gpu, prec):
+    """an infinite relaxation factor leaves NaN everywhere, in the line
+    layout's padding too; a solve from a given start afterwards is a new
+    context's, its measured residual and its stopping test included"""
+    def mk():
+        c = cases.boundary_layer_block(5, 7, 3, dy0=1e-3, growth=1.3, precision=prec, solver="lsgs")
+        c.params.lsgs_max_iter, c.params.lsgs_abs_tol, c.params.lsgs_rel_tol = 30, 0.0, 1e-2
+        g = FlowPsi(c.mesh, c.params)
+        g.set_lines(c.lines)
+        g.set_state(*c.initial_state(g.geometry()["cellcenter"]))
+        return g
+
+    g, f = mk(), mk()
+    x0 = 1e-3 * np.random.default_rng(1).standard_normal((g.ncells, 5))
+    p = g.params
+    w, p.lsgs_relaxation = p.lsgs_relaxation, np.inf
+    g.set_params(p)
+    g.residual()
+    g.assemble()
+    assert np.isnan(g.linear_solve()).any()
+    p.lsgs_relaxation = w
+    g.set_params(p)
+    out = []
+    for s in (g, f):
+        s.residual()
+        s.assemble()
+        out.append(s.linear_solve(x0, info=True))
+    (dg, ig), (df, jf) = out
+    assert 0 < jf["iterations"] < 30 and np.isfinite(jf["resid"])
+    assert ig == jf and np.array_equal(dg, df)
+    f.close(), g.close()
