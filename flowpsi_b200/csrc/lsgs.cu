@@ -24,6 +24,7 @@
 
 #include "fpsi_internal.h"
 #include "kernels.cuh"
+#include "line_quotient.cuh"
 #include "pdl.cuh"
 
 namespace fpsi {
@@ -294,36 +295,6 @@ __device__ __forceinline__ void block_store(T* row, int lane, const T* b) {
 // pivots, [5][32 lanes]; NaN for a pivot outside the range in which
 // quotient() is exact.
 constexpr int DROW = 30 * 32;
-
-// a / b from y = RN(1 / b): the reciprocal's own error is added back
-// (y + yl = 1 / b to twice the precision), so q is within one ulp of a / b,
-// and one correction by its exact remainder rounds it correctly (Markstein's
-// theorem: Computation of elementary functions on the IBM RISC System/6000
-// processor, IBM J. Res. Dev. 34, 1990).  Four dependent FMAs instead of a
-// division's sequence; the result is that of a / b bit for bit while b and a
-// are in the ranges of pivot_ok and tiny() (a zero keeps its value, not its
-// sign).
-template <class T>
-__device__ __forceinline__ T quotient(T a, T b, T y) {
-  const T yl = fma(-b, y, T(1)) * y;
-  const T q = fma(a, y, a * yl);
-  return fma(fma(-b, q, a), y, q);
-}
-// |b| in 2^-100 .. 2^28 (FP32), 2^-300 .. 2^300 (FP64)
-__device__ __forceinline__ bool pivot_ok(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p28f; }
-__device__ __forceinline__ bool pivot_ok(double b) { return fabs(b) >= 0x1p-300 && fabs(b) <= 0x1p300; }
-// the smallest nonzero |a| so far, as a key (twice its bits, less one; zero
-// gives the largest key), and whether one below 2^-90 (2^-600) was among
-// them: there the remainder or the reciprocal's second part may underflow.
-// Above, an overflow ends in a NaN.
-__device__ __forceinline__ uint32_t key_min(uint32_t k, float a) { return min(k, 2u * __float_as_uint(a) - 1u); }
-__device__ __forceinline__ uint32_t key_min(uint32_t k, double a) {
-  return min(k, 2u * uint32_t(__double2hiint(a)) - 1u);
-}
-template <class T>
-__device__ __forceinline__ bool tiny(uint32_t k) {
-  return k < (sizeof(T) == 4 ? 2u * ((127u - 90u) << 23) : 2u * ((1023u - 600u) << 20)) - 1u;
-}
 
 // Gather the line-ordered system: raw diagonal block, in-line couplings
 // (row p to p-1 in L, to p+1 in U), outer couplings and B.  The coupling of
