@@ -2224,11 +2224,12 @@ int fpsi_gnn_predict(fpsi_gnn* m, fpsi_ctx* x, double* x0) {
   if (!m || !x) return FPSI_E_INVALID;
   const int64_t nc = x->H.nc;
   int rc = fpsi::gnn_predict_launch(m, x, x0 ? x->d_stage : nullptr);
-  if (!rc && x0 &&
-      cudaMemcpyAsync(x0, x->d_stage, size_t(nc) * 5 * sizeof(double), cudaMemcpyDeviceToHost, x->stream) != cudaSuccess)
-    rc = FPSI_E_CUDA;
   if (!rc && cudaStreamSynchronize(x->stream) != cudaSuccess) rc = FPSI_E_CUDA;
-  return rc ? rc : take_error(m);
+  if (!rc) rc = take_error(m);
+  if (rc || !x0) return rc;  // a pass that failed leaves the caller's array alone
+  FPSI_CUDA_TRY(cudaMemcpyAsync(x0, x->d_stage, size_t(nc) * 5 * sizeof(double), cudaMemcpyDeviceToHost, x->stream));
+  FPSI_CUDA_TRY(cudaStreamSynchronize(x->stream));
+  return FPSI_OK;
 }
 
 }  // extern "C"

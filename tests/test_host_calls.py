@@ -88,3 +88,30 @@ def mixed():
     g.set_params(p)
 assert made(mixed) == 1
 """)
+
+
+def test_a_failed_inference_leaves_the_callers_array_alone():
+    """a model wait that gave up (its error bit set by the last layer here)"""
+    run("""
+from flowpsi_b200 import _native as N
+from flowpsi_b200.learned import LearnedStart
+c = cases.taylor_green_tets(4, precision="ref")
+g = FlowPsi(c.mesh, c.params)
+g.set_state(*c.initial_state(g.geometry()["cellcenter"]))
+g.residual(); g.assemble()
+m = LearnedStart(seed=0)
+fail = True
+def give_up(c):
+    if fail and c.what == "launch" and "k_layer_ws" in c.name:
+        args = C.cast(c.args, C.POINTER(C.c_void_p))
+        err = C.cast(args[12], C.POINTER(C.c_void_p))[0]  # its last argument, int32_t* err
+        C.cast(err, C.POINTER(C.c_int32))[0] = 2
+    return 0
+on.append(give_up)
+x0 = np.full(g.ncells * 5, 7.0)
+assert N.lib().fpsi_gnn_predict(m._h, g._ctx, N.dptr(x0)) == -7  # FPSI_E_TIMEOUT
+assert (x0 == 7.0).all()
+fail = False
+assert N.lib().fpsi_gnn_predict(m._h, g._ctx, N.dptr(x0)) == 0
+assert not (x0 == 7.0).any()
+""")
