@@ -1021,7 +1021,6 @@ static int launch_thomas(fpsi_ctx* x, int64_t g0, int64_t ng, bool use_B, const 
   }
   auto k = ylen > 0 ? dev::k_lsgs_thomas<TB, TD, TX, true> : dev::k_lsgs_thomas<TB, TD, TX, false>;
   const size_t smem = dev::thomas_smem_bytes<TB, TD, TX>(nst, ylen);
-  FPSI_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   prof_begin(x, "lsgs_thomas");
   launch_chain(x, k, ng, dev::THOMAS_THREADS, smem, nst, g0, line_view(x), (const TD*)x->d_lD, (const TB*)x->d_lL, (const TB*)x->d_lU, (TX*)x->d_lrhs,
       (const TB*)x->d_lB, use_B, (TX*)x->d_lx, ctl, x->d_err);
@@ -1038,6 +1037,10 @@ static int lsgs_solve_t(fpsi_ctx* x, bool jacobi_start) {
   const int64_t nt = Y.nrows * 32;
   TX* X = (TX*)x->d_lx;
   TX* XT = (TX*)x->d_lxt;
+  // A limit, the same for every context and thread: one that followed the
+  // launch's own size could be lowered by another's between here and there.
+  for (auto k : {dev::k_lsgs_thomas<TB, TD, TX, true>, dev::k_lsgs_thomas<TB, TD, TX, false>})
+    FPSI_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dev::THOMAS_SMEM_MAX)));
   // in full: the launches behind it read the system before their waits
   dev::k_lsgs_init<<<1, 1, 0, s>>>(ctl, x->P.lsgs_relaxation);
   int rc;

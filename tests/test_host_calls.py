@@ -115,3 +115,44 @@ fail = False
 assert N.lib().fpsi_gnn_predict(m._h, g._ctx, N.dptr(x0)) == 0
 assert not (x0 == 7.0).any()
 """)
+
+
+def test_line_solves_share_one_shared_memory_limit():
+    """the limit belongs to the kernel, not to a context: two contexts with
+    lines of different lengths, and colours with more and with fewer groups
+    than the device has multiprocessors, all launch under one value"""
+    run("""
+from flowpsi_b200.solver import GeneratedMesh, bc
+from tests.test_gpu_line_groups import uneven_lines
+limit, need, above = {}, {}, []
+def look(c):
+    if "k_lsgs_thomas" in c.name:
+        if c.what == "attribute":
+            limit.setdefault(c.name, set()).add(c.n)
+        if c.what == "launch":
+            if c.n > min(limit[c.name]):
+                above.append(c)
+            need.setdefault(c.name, set()).add(c.n)
+    return 0
+on.append(look)
+def solver(n, prec):
+    mesh = GeneratedMesh("hex", n=n, bc_side=(0,) * 6, bcs=[bc("farfield")])
+    p = cases.farfield_cube(2, precision=prec).params
+    p.solver, p.lsgs_max_iter = 1, 2
+    g = FlowPsi(mesh, p)
+    g.set_state(np.full(g.ncells, 300.0), np.full(g.ncells, 1e5), np.zeros((g.ncells, 3)))
+    return g, mesh
+def use(g):
+    g.residual(); g.assemble(); g.linear_solve()
+for prec in ("mixed", "ref", "fp64"):
+    a, ma = solver((4, 600, 2), prec)   # too long for shared memory
+    a.set_lines(ma.lines_along(1))
+    b, mb = solver((110, 2, 110), prec)
+    b.set_lines(uneven_lines(mb, 110))
+    for s in (a, b, a, b):
+        use(s)
+    a.close(), b.close()
+assert not above, above[0]
+assert len(need) == 6 and max(len(v) for v in need.values()) > 1, need
+assert all(len(v) == 1 for v in limit.values()), limit
+""")
