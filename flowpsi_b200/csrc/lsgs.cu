@@ -703,6 +703,9 @@ k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* lD, const TB* lL,
     return;
   }
 
+  // the walking warp goes on or gives up as one: the votes and barriers of its
+  // loops need every lane
+  auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
   static_assert(sizeof(TD) == sizeof(TX), "the factors and the iterate have one type");
   // register sets: the next row's blocks beside this one's, except where both
   // are FP64 (they would spill)
@@ -739,7 +742,7 @@ k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* lD, const TB* lL,
   // on to the next chunk's stage; release: hands one back
   auto advance = [&]() {
     if (++s == nst) s = 0, parity ^= 1;
-    ok = wait(full + s, parity) && ok;
+    ok = wait_all(full + s, parity) && ok;
   };
   auto release = [&](int st) {
     __syncwarp();
@@ -863,7 +866,7 @@ k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* lD, const TB* lL,
   using no = std::false_type;
   if (nch > 0) {
     const int nfull = glen / R;
-    ok = wait(full, 0);
+    ok = wait_all(full, 0);
     if (NS == 2) fetch(0, 0, 0, true);
     for (int c = 0; c < nfull && ok; ++c) chunk(c, yes{}, yes{}, c + 1 < nch);
     if (nfull < nch && ok) chunk(nfull, no{}, yes{}, false);
