@@ -53,6 +53,14 @@ int dalloc(fpsi_ctx* x, T** p, size_t n) {
   return FPSI_OK;
 }
 
+// Set-up runs on the default stream, which the contexts' streams do not wait
+// for (nor does a copy from pageable memory, or a memset, wait to be done):
+// waited for here before the context is used.
+int settle() {
+  FPSI_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return FPSI_OK;
+}
+
 template <class T>
 int upload(fpsi_ctx* x, T** p, const std::vector<T>& h) {
   int rc = dalloc(x, p, h.size());
@@ -151,7 +159,7 @@ int alloc_sa(fpsi_ctx* x) {
   std::vector<double> v(nc, 1e-6);
   FPSI_CUDA_TRY(cudaMemcpy(x->d_nut, v.data(), nc * sizeof(double), cudaMemcpyHostToDevice));
   FPSI_CUDA_TRY(cudaMemcpy(x->d_wdist, x->h_wdist.data(), nc * sizeof(double), cudaMemcpyHostToDevice));
-  return FPSI_OK;
+  return settle();
 }
 
 int alloc_lsgs(fpsi_ctx* x) {
@@ -191,7 +199,7 @@ int alloc_lsgs(fpsi_ctx* x) {
   FPSI_CUDA_TRY(cudaMemset(x->d_lB, 0, nt * 5 * tb));
   x->lsgs_prec = x->P.precision;
   x->keep_D = true;  // the line preprocessing starts from the unfactored blocks
-  return FPSI_OK;
+  return settle();
 }
 
 // residual history for runs of up to n steps
@@ -531,6 +539,7 @@ int fpsi_create(fpsi_ctx** out, const fpsi_mesh* mesh, const fpsi_params* params
   TRY(alloc_lsgs(x));
   fpsi::wall_distance(mesh, x->H, x->h_wdist);
   TRY(alloc_sa(x));
+  TRY(settle());
 #undef TRY
   *out = x;
   return FPSI_OK;
@@ -809,7 +818,7 @@ static int finish_assemble(fpsi_ctx* x) {
   int rc = sync(x);
   if (rc) return rc;
   if (err) {
-    FPSI_CUDA_TRY(cudaMemset(x->d_err, 0, sizeof(int32_t)));
+    FPSI_CUDA_TRY(cudaMemsetAsync(x->d_err, 0, sizeof(int32_t), x->stream));
     if (err & 4) {
       fpsi::set_error("a line solve gave up waiting for its staged rows");
       return FPSI_E_TIMEOUT;
@@ -1038,7 +1047,7 @@ int fpsi_newton_step(fpsi_ctx* x, fpsi_stepinfo* info) {
   if (has_nan(x->h_resid)) {
     // the state was left unchanged; a system built from NaN norms may have
     // flagged zero pivots too
-    FPSI_CUDA_TRY(cudaMemset(x->d_err, 0, sizeof(int32_t)));
+    FPSI_CUDA_TRY(cudaMemsetAsync(x->d_err, 0, sizeof(int32_t), x->stream));
     fpsi::set_error("NaN residual norms; the state is unchanged");
     return FPSI_E_NAN;
   }
@@ -1303,7 +1312,7 @@ static int finish_run(fpsi_ctx* x, int32_t nsteps, int32_t launched, fpsi_resid*
   }
   if (first_nan >= 0) {
     // the systems built from NaN norms may have flagged zero pivots too
-    FPSI_CUDA_TRY(cudaMemset(x->d_err, 0, sizeof(int32_t)));
+    FPSI_CUDA_TRY(cudaMemsetAsync(x->d_err, 0, sizeof(int32_t), x->stream));
     fpsi::set_error("NaN residual norms at step %d of %d; the state is that step's", first_nan,
                     nsteps);
     return FPSI_E_NAN;

@@ -1544,7 +1544,8 @@ int take_error(fpsi_gnn* m) {
   int32_t e = 0;
   FPSI_CUDA_TRY(cudaMemcpy(&e, m->d_err, sizeof(e), cudaMemcpyDeviceToHost));
   if (!e) return FPSI_OK;
-  FPSI_CUDA_TRY(cudaMemset(m->d_err, 0, sizeof(int32_t)));
+  FPSI_CUDA_TRY(cudaMemsetAsync(m->d_err, 0, sizeof(int32_t), m->stream));
+  FPSI_CUDA_TRY(cudaStreamSynchronize(m->stream));  // an inference runs on its context's stream
   fpsi::set_error("learned start: a tensor-core wait timed out");
   return FPSI_E_TIMEOUT;
 }
@@ -1680,6 +1681,8 @@ int ctx_graph(fpsi_ctx* x, Graph* G) {
     FPSI_CUDA_TRY(cudaMemcpy(x->d_cnb_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice));
     if (!nb.empty())
       FPSI_CUDA_TRY(cudaMemcpy(x->d_cnb, nb.data(), nb.size() * 4, cudaMemcpyHostToDevice));
+    // on the default stream, which the streams that read them do not wait for
+    FPSI_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     x->cnb_n = int64_t(nb.size());
   }
   *G = Graph{nc, x->d_cnb_off, x->d_cnb, x->d_enb, x->H.ell_k};
@@ -1721,7 +1724,7 @@ int fpsi_gnn_create(fpsi_gnn** out, uint64_t seed) {
   G(galloc(&m->d_err, 1));
   G(galloc(&m->d_fac, 64));
 #undef G
-  if (!rc && cudaMemset(m->d_err, 0, sizeof(int32_t)) != cudaSuccess) rc = FPSI_E_CUDA;
+  if (!rc && cudaMemsetAsync(m->d_err, 0, sizeof(int32_t), m->stream) != cudaSuccess) rc = FPSI_E_CUDA;
   int dev = 0;
   if (!rc && (cudaGetDevice(&dev) != cudaSuccess ||
               cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -1809,9 +1812,9 @@ int fpsi_gnn_get_params(fpsi_gnn* m, float* w) {
 
 int fpsi_gnn_set_params(fpsi_gnn* m, const float* w) {
   if (!m || !w) return FPSI_E_INVALID;
-  FPSI_CUDA_TRY(cudaMemcpy(m->d_w, w, m->L.total * 4, cudaMemcpyHostToDevice));
-  FPSI_CUDA_TRY(cudaMemset(m->d_m, 0, m->L.total * 4));
-  FPSI_CUDA_TRY(cudaMemset(m->d_v, 0, m->L.total * 4));
+  FPSI_CUDA_TRY(cudaMemcpyAsync(m->d_w, w, m->L.total * 4, cudaMemcpyHostToDevice, m->stream));
+  FPSI_CUDA_TRY(cudaMemsetAsync(m->d_m, 0, m->L.total * 4, m->stream));
+  FPSI_CUDA_TRY(cudaMemsetAsync(m->d_v, 0, m->L.total * 4, m->stream));
   m->adam_t = 0;
   k_to_bf16<<<nb_(m->L.total, 256), 256, 0, m->stream>>>(m->L.total, m->d_w, m->d_wb);
   FPSI_CUDA_TRY(cudaStreamSynchronize(m->stream));

@@ -156,3 +156,57 @@ assert not above, above[0]
 assert len(need) == 6 and max(len(v) for v in need.values()) > 1, need
 assert all(len(v) == 1 for v in limit.values()), limit
 """)
+
+
+def test_set_up_on_the_default_stream_is_waited_for():
+    """the contexts' and models' streams do not wait for the default stream: a
+    clear or an upload on it is complete before either stream is given work"""
+    run("""
+from flowpsi_b200.learned import LearnedStart
+pending, early = [], []
+def look(c):
+    if c.what in ("memset", "copy_up"):
+        pending.append(c)
+    elif c.what in ("copy_down", "sync_device") or (c.what == "sync" and c.stream <= 1):
+        pending.clear()
+    elif c.stream > 1 and c.what != "sync" and pending:
+        early.append((pending[-1][:6], c[:6]))
+        pending.clear()
+    return 0
+on.append(look)
+def step(what):
+    assert not early, (what, early[0])
+
+c = cases.boundary_layer_block(4, 6, 3, dy0=1e-3, growth=1.3, viscous=2, precision="ref", sa=True)
+g = FlowPsi(c.mesh, c.params)
+st = c.initial_state(g.geometry()["cellcenter"])
+g.set_state(*st); step("create")
+g.residual(); g.set_lines(c.lines); g.assemble(); g.linear_solve(); step("lines")
+c = cases.taylor_green_tets(4, precision="ref")
+g = FlowPsi(c.mesh, c.params)
+g.set_state(*c.initial_state(g.geometry()["cellcenter"]))
+p = g.params
+p.viscous, p.turbulence = 2, 1
+g.set_params(p); g.residual(); step("SA switched on")
+p.viscous = p.turbulence = 0; p.solver = 1
+g.set_params(p); g.residual(); g.assemble(); g.linear_solve(); step("line solver switched on")
+p.solver = 0
+g.set_params(p); g.residual(); g.assemble()
+m = LearnedStart(seed=0); step("model")
+m.predict(g); step("inference")
+m.set_params(m.get_params()); m.add_snapshot(g, np.zeros((g.ncells, 5))); m.train(2); step("training")
+
+# the error bits, cleared after a failure
+def zero_pivot(c):
+    if c.what == "copy_down_async" and c.n == 4:  # of the assembly's error bits
+        C.cast(c.q, C.POINTER(C.c_int32))[0] = 1
+    return 0
+on.append(zero_pivot)
+try:
+    g.residual(); g.assemble()
+    raise SystemExit("no error")
+except FpsiError:
+    pass
+on.remove(zero_pivot)
+g.residual(); g.assemble(); step("after a zero pivot")
+""")
