@@ -46,6 +46,7 @@ int dalloc(fpsi_ctx* x, T** p, size_t n) {
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
   if (e != cudaSuccess) {
     fpsi::set_error("cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
+    cudaGetLastError();
     *p = nullptr;
     return e == cudaErrorMemoryAllocation ? FPSI_E_NOMEM : FPSI_E_CUDA;
   }
@@ -210,6 +211,7 @@ int ensure_hist(fpsi_ctx* x, int64_t n) {
   x->hist_cap = 0;
   if (cudaMallocHost((void**)&x->h_hist, size_t(n) * fpsi::NREC * sizeof(double)) != cudaSuccess) {
     fpsi::set_error("cudaMallocHost of the residual history failed");
+    cudaGetLastError();
     return FPSI_E_NOMEM;
   }
   x->hist_cap = n;

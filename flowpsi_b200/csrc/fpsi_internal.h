@@ -33,6 +33,7 @@ void set_error(const char* fmt, ...);
     cudaError_t e_ = (expr);                                                         \
     if (e_ != cudaSuccess) {                                                         \
       ::fpsi::set_error("%s:%d %s: %s", __FILE__, __LINE__, #expr, cudaGetErrorString(e_)); \
+      cudaGetLastError(); /* reported here, not by the next call too */               \
       return FPSI_E_CUDA;                                                            \
     }                                                                                \
   } while (0)

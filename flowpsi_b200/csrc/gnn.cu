@@ -1554,6 +1554,7 @@ template <class T>
 int galloc(T** p, size_t n) {
   if (cudaMalloc((void**)p, (n ? n : 1) * sizeof(T)) != cudaSuccess) {
     fpsi::set_error("cudaMalloc failed in the learned-start model");
+    cudaGetLastError();
     *p = nullptr;
     return FPSI_E_NOMEM;
   }
@@ -1835,6 +1836,7 @@ static int make_features(fpsi_gnn* m, fpsi_ctx* x, float* feat, float* xj, float
     if (cudaMalloc(&x->d_xprev, size_t(nc) * 5 * 8) != cudaSuccess) {
       x->d_xprev = nullptr;
       fpsi::set_error("cudaMalloc failed for the previous-update copy");
+      cudaGetLastError();
       return FPSI_E_NOMEM;
     }
     x->have_xprev = false;
@@ -2258,6 +2260,7 @@ int gnn_predict_launch(fpsi_gnn* m, fpsi_ctx* x, double* dx0, bool jacobi_in_ite
     if (cudaMalloc(&x->d_xprev, size_t(nc) * 5 * 8) != cudaSuccess) {
       x->d_xprev = nullptr;
       set_error("cudaMalloc failed for the previous-update copy");
+      cudaGetLastError();
       return FPSI_E_NOMEM;
     }
     x->have_xprev = false;

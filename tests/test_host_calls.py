@@ -210,3 +210,35 @@ except FpsiError:
 on.remove(zero_pivot)
 g.residual(); g.assemble(); step("after a zero pivot")
 """)
+
+
+def test_an_error_is_reported_once():
+    """a call that the runtime refused leaves nothing behind that makes the
+    next call fail"""
+    run("""
+c = cases.farfield_cube(4, precision="ref")
+g = FlowPsi(c.mesh, c.params)
+st = c.initial_state(g.geometry()["cellcenter"])
+def refuse(c):
+    return 2 if c.what == "copy_up_async" else 0  # cudaErrorMemoryAllocation
+on.append(refuse)
+try:
+    g.set_state(*st)
+    raise SystemExit("no error")
+except FpsiError:
+    pass
+on.remove(refuse)
+g.set_state(*st)
+g.residual()
+# nor another context's allocation
+def full(c):
+    return 2 if c.what == "malloc" else 0
+on.append(full)
+try:
+    FlowPsi(c.mesh, c.params)
+    raise SystemExit("no error")
+except FpsiError:
+    pass
+on.remove(full)
+g.residual()
+""")
