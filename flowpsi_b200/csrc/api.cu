@@ -1488,7 +1488,9 @@ struct Batch {
   char* p = nullptr;
   double *L = nullptr, *R = nullptr, *A = nullptr, *S = nullptr;
   void* out = nullptr;
+  bool queued = false;  // copies to or from the caller's arrays may be in flight
   ~Batch() {
+    if (queued) cudaStreamSynchronize(s);  // a call that failed on its way
     if (p) cudaFreeAsync(p, s);
   }
   int put(int64_t n, const double* qL, const double* qR, const double* an, const double* area, size_t out_bytes) {
@@ -1516,6 +1518,7 @@ struct Batch {
       return e == cudaErrorMemoryAllocation ? FPSI_E_NOMEM : FPSI_E_CUDA;
     }
     L = (double*)(p + oL), R = (double*)(p + oR), A = (double*)(p + oA), S = (double*)(p + oS), out = p + oO;
+    queued = true;
     FPSI_CUDA_TRY(cudaMemcpyAsync(L, qL, n * 5 * d, cudaMemcpyHostToDevice, s));
     FPSI_CUDA_TRY(cudaMemcpyAsync(R, qR, n * 5 * d, cudaMemcpyHostToDevice, s));
     FPSI_CUDA_TRY(cudaMemcpyAsync(A, an, n * 3 * d, cudaMemcpyHostToDevice, s));
@@ -1524,6 +1527,7 @@ struct Batch {
   }
   int get(void* host, size_t bytes) {
     FPSI_CUDA_TRY(cudaMemcpyAsync(host, out, bytes, cudaMemcpyDeviceToHost, s));
+    queued = false;
     FPSI_CUDA_TRY(cudaStreamSynchronize(s));
     return FPSI_OK;
   }

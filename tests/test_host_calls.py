@@ -242,3 +242,36 @@ except FpsiError:
 on.remove(full)
 g.residual()
 """)
+
+
+def test_a_failed_face_call_waits_for_its_copies():
+    """no copy from the caller's arrays is left in flight when a batched face
+    call returns an error, whichever of its calls failed"""
+    run("""
+from flowpsi_b200 import inviscid_riemann_flux, roe_jacobian
+from tests.helpers import face_states
+faces = face_states(10, 0)
+def fail(what, k):
+    n = [0]
+    def f(c):
+        if c.what != what:
+            return 0
+        n[0] += 1
+        return 700 if n[0] == k else 0
+    return f
+for call in (lambda: inviscid_riemann_flux("roe", *faces), lambda: roe_jacobian(*faces, 1)):
+    call()
+    for what, k in (("copy_up_async", 2), ("copy_up_async", 4), ("launch", 1), ("copy_down_async", 1)):
+        del calls[:]
+        on.append(fail(what, k))
+        try:
+            call()
+            raise SystemExit("no error")
+        except FpsiError:
+            pass
+        del on[:]
+        ups = [i for i, c in enumerate(calls) if c.what == "copy_up_async"]
+        waits = [i for i, c in enumerate(calls) if c.what == "sync" and c.stream == calls[ups[0]].stream]
+        assert waits and waits[-1] > ups[-1], (what, k, [c.what for c in calls])
+        assert sum(c.what == "malloc_pool" for c in calls) == sum(c.what == "free_pool" for c in calls)
+""")
