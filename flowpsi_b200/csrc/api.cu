@@ -302,6 +302,14 @@ void unpermute_cells(const fpsi_ctx* x, const T* dev_order, int w, T* caller) {
   }
 }
 
+// the end of a call that may have queued copies of the caller's arrays: they
+// are not in flight any more when it returns, with an error neither
+int finish(fpsi_ctx* x, int rc) {
+  if (!rc) return sync(x);
+  cudaStreamSynchronize(x->stream);
+  return rc;
+}
+
 // per-cell device rows (w <= 5 values) into a caller-order host array, and
 // back: permuted on the device through the staging buffer
 int rows_down(fpsi_ctx* x, int w, const int32_t* map, const void* src, int bytes, double* out) {
@@ -314,8 +322,7 @@ int rows_down(fpsi_ctx* x, int w, const int32_t* map, const void* src, int bytes
 int rows_up(fpsi_ctx* x, int w, const int32_t* map, const double* in, void* dst, int bytes) {
   FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage, in, size_t(x->H.nc) * w * sizeof(double), cudaMemcpyHostToDevice,
                                 x->stream));
-  const int rc = fpsi::launch_rows_in(x, w, map, x->d_stage, dst, bytes);
-  return rc ? rc : sync(x);
+  return finish(x, fpsi::launch_rows_in(x, w, map, x->d_stage, dst, bytes));
 }
 
 }  // namespace
@@ -738,26 +745,32 @@ int fpsi_set_state(fpsi_ctx* x, const double* T, const double* pg, const double*
   if (!x || !T || !pg || !u) return FPSI_E_INVALID;
   const int64_t nc = x->H.nc;
   const size_t b = size_t(nc) * sizeof(double);
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage, T, b, cudaMemcpyHostToDevice, x->stream));
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage + nc, pg, b, cudaMemcpyHostToDevice, x->stream));
-  FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage + 2 * nc, u, 3 * b, cudaMemcpyHostToDevice, x->stream));
-  int rc = fpsi::launch_state(x, true);
-  if (rc) return rc;
-  x->have_resid = x->have_asm = x->have_dq = x->have_xprev = false;
-  x->have_levels = false;
-  return sync(x);
+  auto queue = [&]() -> int {
+    FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage, T, b, cudaMemcpyHostToDevice, x->stream));
+    FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage + nc, pg, b, cudaMemcpyHostToDevice, x->stream));
+    FPSI_CUDA_TRY(cudaMemcpyAsync(x->d_stage + 2 * nc, u, 3 * b, cudaMemcpyHostToDevice, x->stream));
+    const int rc = fpsi::launch_state(x, true);
+    if (rc) return rc;
+    x->have_resid = x->have_asm = x->have_dq = x->have_xprev = false;
+    x->have_levels = false;
+    return FPSI_OK;
+  };
+  return finish(x, queue());
 }
 
 int fpsi_get_state(fpsi_ctx* x, double* T, double* pg, double* u) {
   if (!x || !T || !pg || !u) return FPSI_E_INVALID;
   const int64_t nc = x->H.nc;
   const size_t b = size_t(nc) * sizeof(double);
-  int rc = fpsi::launch_state(x, false);
-  if (rc) return rc;
-  FPSI_CUDA_TRY(cudaMemcpyAsync(T, x->d_stage, b, cudaMemcpyDeviceToHost, x->stream));
-  FPSI_CUDA_TRY(cudaMemcpyAsync(pg, x->d_stage + nc, b, cudaMemcpyDeviceToHost, x->stream));
-  FPSI_CUDA_TRY(cudaMemcpyAsync(u, x->d_stage + 2 * nc, 3 * b, cudaMemcpyDeviceToHost, x->stream));
-  return sync(x);
+  auto queue = [&]() -> int {
+    const int rc = fpsi::launch_state(x, false);
+    if (rc) return rc;
+    FPSI_CUDA_TRY(cudaMemcpyAsync(T, x->d_stage, b, cudaMemcpyDeviceToHost, x->stream));
+    FPSI_CUDA_TRY(cudaMemcpyAsync(pg, x->d_stage + nc, b, cudaMemcpyDeviceToHost, x->stream));
+    FPSI_CUDA_TRY(cudaMemcpyAsync(u, x->d_stage + 2 * nc, 3 * b, cudaMemcpyDeviceToHost, x->stream));
+    return FPSI_OK;
+  };
+  return finish(x, queue());
 }
 
 int fpsi_keep_blocks(fpsi_ctx* x, int32_t keep) {

@@ -1910,9 +1910,11 @@ int fpsi_gnn_add_snapshot(fpsi_gnn* m, fpsi_ctx* x, const double* dq) {
             cudaMemcpyAsync(dscl, s.xs, 5 * sizeof(float), cudaMemcpyHostToDevice, m->stream) == cudaSuccess;
   if (ok) {
     k_target<<<nb_(nc * 5, 256), 256, 0, m->stream>>>(nc, dd, x->d_perm, s.xj, dscl, s.target);
-    ok = cudaStreamSynchronize(m->stream) == cudaSuccess;
+    ok = cudaGetLastError() == cudaSuccess;
   }
+  ok = cudaStreamSynchronize(m->stream) == cudaSuccess && ok;  // dq is not read any more, after an error neither
   if (!ok) {
+    cudaGetLastError();
     free_snapshot(s);
     fpsi::set_error("learned start: snapshot upload failed");
     return FPSI_E_CUDA;

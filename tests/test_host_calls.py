@@ -275,3 +275,59 @@ for call in (lambda: inviscid_riemann_flux("roe", *faces), lambda: roe_jacobian(
         assert waits and waits[-1] > ups[-1], (what, k, [c.what for c in calls])
         assert sum(c.what == "malloc_pool" for c in calls) == sum(c.what == "free_pool" for c in calls)
 """)
+
+
+def test_a_failed_call_leaves_no_copy_of_the_callers_arrays_in_flight():
+    """each call that moves an array between the caller and the device, with
+    each of its copies and launches refused in turn: whatever it queued has
+    been waited for when it returns the error"""
+    run("""
+from flowpsi_b200.learned import LearnedStart
+STREAM = ("copy_up_async", "copy_down_async", "copy_async", "launch")
+c = cases.taylor_green_tets(4, precision="ref")
+c.params.viscous, c.params.turbulence = 2, 1
+g = FlowPsi(c.mesh, c.params)
+st = c.initial_state(g.geometry()["cellcenter"])
+v1, v5 = np.ones(g.ncells), np.zeros((g.ncells, 5))
+m = LearnedStart(seed=0)
+def ready(sa):
+    p = g.params
+    p.viscous, p.turbulence = (2, 1) if sa else (0, 0)
+    g.set_params(p)
+    g.set_state(*st); g.residual(); g.assemble()
+tried = 0
+for name, sa, f in [
+        ("set_state", 1, lambda: g.set_state(*st)), ("get_state", 1, lambda: g.get_state()),
+        ("set_eddy_viscosity", 1, lambda: g.set_eddy_viscosity(v1)), ("eddy_viscosity", 1, lambda: g.eddy_viscosity()),
+        ("set_nutilde", 1, lambda: g.set_nutilde(v1)), ("nutilde", 1, lambda: g.nutilde()),
+        ("residual", 0, lambda: g.residual()), ("dtau", 0, lambda: g.dtau()),
+        ("linear_solve", 0, lambda: g.linear_solve(v5)), ("set_iterate", 0, lambda: g.set_iterate(v5)),
+        ("get_iterate", 0, lambda: g.get_iterate()), ("predict", 0, lambda: m.predict(g, want=True)),
+        ("add_snapshot", 0, lambda: m.add_snapshot(g, v5))]:
+    ready(sa)
+    f()
+    for k in range(1, 100):
+        ready(sa)
+        del calls[:]
+        n = [0]
+        def refuse(c):
+            n[0] += c.what in STREAM
+            return 700 if c.what in STREAM and n[0] == k else 0
+        on.append(refuse)
+        try:
+            f()
+            failed = False
+        except FpsiError:
+            failed = True
+        on.remove(refuse)
+        if n[0] < k:
+            break
+        assert failed, (name, k)
+        tried += 1
+        seen = 0
+        for i, c in enumerate(calls):
+            seen += c.what in STREAM
+            if c.what in ("copy_up_async", "copy_down_async") and seen != k:
+                assert any(d.what == "sync" and d.stream == c.stream for d in calls[i:]), (name, k, c)
+assert tried > 30, tried
+""")
