@@ -35,23 +35,35 @@ void prof_end(fpsi_ctx* x) {
   if (!x->profiling || x->prof.empty()) return;
   cudaEventRecord(x->prof.back().b, x->stream);
 }
+
+int device_alloc(fpsi_ctx* x, void** p, size_t bytes) {
+  *p = nullptr;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    set_error("cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+    cudaGetLastError();
+    *p = nullptr;
+    return e == cudaErrorMemoryAllocation ? FPSI_E_NOMEM : FPSI_E_CUDA;
+  }
+  x->held[*p] = int64_t(bytes);
+  x->device_bytes += int64_t(bytes);
+  return FPSI_OK;
+}
+void device_free(fpsi_ctx* x, void* p) {
+  if (!p) return;
+  cudaFree(p);
+  const auto it = x->held.find(p);
+  if (it == x->held.end()) return;
+  x->device_bytes -= it->second;
+  x->held.erase(it);
+}
 }  // namespace fpsi
 
 namespace {
 
 template <class T>
 int dalloc(fpsi_ctx* x, T** p, size_t n) {
-  *p = nullptr;
-  if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
-  if (e != cudaSuccess) {
-    fpsi::set_error("cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
-    cudaGetLastError();
-    *p = nullptr;
-    return e == cudaErrorMemoryAllocation ? FPSI_E_NOMEM : FPSI_E_CUDA;
-  }
-  x->device_bytes += int64_t(n * sizeof(T));
-  return FPSI_OK;
+  return fpsi::device_alloc(x, (void**)p, (n ? n : 1) * sizeof(T));
 }
 
 // Set-up runs on the default stream, which the contexts' streams do not wait
@@ -81,8 +93,7 @@ std::vector<double> soa3(const std::vector<double>& a, int64_t n) {
 void free_system(fpsi_ctx* x) {
   void* ps[] = {x->d_fjp, x->d_fjm, x->d_fjc, x->d_D, x->d_x, x->d_luc, x->d_bc, x->d_pv, x->d_aoff,
                 x->d_bjac};
-  for (void* p : ps)
-    if (p) cudaFree(p);
+  for (void* p : ps) fpsi::device_free(x, p);
   x->d_fjp = x->d_fjm = x->d_fjc = x->d_D = x->d_x = x->d_luc = x->d_bc = x->d_aoff = nullptr;
   x->d_bjac = nullptr;
   x->d_pv = nullptr;
@@ -119,8 +130,7 @@ int alloc_system(fpsi_ctx* x) {
 void free_lsgs(fpsi_ctx* x) {
   void* ps[] = {x->d_lt, x->d_lct, x->d_lonbr, x->d_llen, x->d_lrole, x->d_lrow0, x->d_lD, x->d_lL,
                 x->d_lU, x->d_lF, x->d_lB, x->d_lrhs, x->d_lx, x->d_lxt, x->d_lctl, x->d_lpart};
-  for (void* p : ps)
-    if (p) cudaFree(p);
+  for (void* p : ps) fpsi::device_free(x, p);
   x->d_lt = x->d_lct = x->d_lonbr = x->d_llen = nullptr;
   x->d_lrole = nullptr;
   x->d_lrow0 = nullptr;
@@ -134,8 +144,7 @@ void free_lsgs(fpsi_ctx* x) {
 void free_sa(fpsi_ctx* x) {
   double* ps[] = {x->d_nut, x->d_wdist, x->d_sa_grad, x->d_sa_phi, x->d_sa_nub,
                   x->d_sa_face, x->d_sa_B, x->d_sa_D, x->d_sa_Dinv, x->d_sa_x};
-  for (double* p : ps)
-    if (p) cudaFree(p);
+  for (double* p : ps) fpsi::device_free(x, p);
   x->d_nut = x->d_wdist = x->d_sa_grad = x->d_sa_phi = x->d_sa_nub = nullptr;
   x->d_sa_face = x->d_sa_B = x->d_sa_D = x->d_sa_Dinv = x->d_sa_x = nullptr;
   x->have_sa = x->have_sa_dq = false;
@@ -404,8 +413,7 @@ int fpsi_destroy(fpsi_ctx* x) {
                 x->d_qn, x->d_qnm1, x->d_qb, x->d_grad, x->d_qf, x->d_F, x->d_src, x->d_dtau, x->d_tmu, x->d_muk,
                 x->d_part, x->d_resid, x->d_amin, x->d_err, x->d_perm, x->d_stage, x->d_ci, x->d_ccol,
                 x->d_nbr, x->d_colinfo, x->d_cnb_off, x->d_cnb, x->d_xprev, x->d_qsave, x->d_adiss, x->d_ageom};
-  for (void* p : ps)
-    if (p) cudaFree(p);
+  for (void* p : ps) fpsi::device_free(x, p);
   if (x->h_resid) cudaFreeHost(x->h_resid);
   if (x->h_flags) cudaFreeHost(x->h_flags);
   if (x->h_amin) cudaFreeHost(x->h_amin);

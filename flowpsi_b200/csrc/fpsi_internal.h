@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/fpsi.h"
@@ -229,7 +230,8 @@ struct fpsi_ctx {
   double *d_sa_nub = nullptr, *d_sa_face = nullptr;  // [nbf], [7][nf]
   double *d_sa_B = nullptr, *d_sa_D = nullptr, *d_sa_Dinv = nullptr, *d_sa_x = nullptr;
   bool have_sa = false, have_sa_dq = false;
-  int64_t device_bytes = 0;
+  int64_t device_bytes = 0;  // of the allocations below
+  std::unordered_map<void*, int64_t> held;
   // caller-order staging for state transfers (T, pg, u) and the permutation
   int32_t* d_perm = nullptr;   // new cell id -> caller cell id
   double* d_stage = nullptr;   // [nc] T, [nc] pg, [3 nc] u (caller order)
@@ -254,6 +256,9 @@ struct fpsi_ctx {
 namespace fpsi {
 void prof_begin(fpsi_ctx* x, const char* name);
 void prof_end(fpsi_ctx* x);
+// device memory of a context, counted in what fpsi_info reports
+int device_alloc(fpsi_ctx* x, void** p, size_t bytes);
+void device_free(fpsi_ctx* x, void* p);
 // line SGS: layout from caller lines (RCM ids) or the default rule
 int build_lines(fpsi_ctx* x, const std::vector<std::vector<int32_t>>* lines);
 int lsgs_assemble(fpsi_ctx* x);

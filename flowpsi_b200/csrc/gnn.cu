@@ -1672,10 +1672,10 @@ int ctx_graph(fpsi_ctx* x, Graph* G) {
       }
       off[c + 1] = int32_t(nb.size());
     }
-    int rc = galloc(&x->d_cnb_off, off.size());
-    if (!rc) rc = galloc(&x->d_cnb, nb.size());
+    int rc = fpsi::device_alloc(x, (void**)&x->d_cnb_off, off.size() * sizeof(int32_t));
+    if (!rc) rc = fpsi::device_alloc(x, (void**)&x->d_cnb, std::max<size_t>(nb.size(), 1) * sizeof(int32_t));
     if (rc) {
-      cudaFree(x->d_cnb_off), cudaFree(x->d_cnb);
+      fpsi::device_free(x, x->d_cnb_off), fpsi::device_free(x, x->d_cnb);
       x->d_cnb_off = x->d_cnb = nullptr;
       return rc;
     }
@@ -1833,12 +1833,8 @@ static int make_features(fpsi_gnn* m, fpsi_ctx* x, float* feat, float* xj, float
   if (nc > m->cap) return FPSI_E_INVALID;
   // from now on the context keeps a copy of each applied update
   if (!x->d_xprev) {
-    if (cudaMalloc(&x->d_xprev, size_t(nc) * 5 * 8) != cudaSuccess) {
-      x->d_xprev = nullptr;
-      fpsi::set_error("cudaMalloc failed for the previous-update copy");
-      cudaGetLastError();
-      return FPSI_E_NOMEM;
-    }
+    const int rc = fpsi::device_alloc(x, (void**)&x->d_xprev, size_t(nc) * 5 * 8);
+    if (rc) return rc;
     x->have_xprev = false;
   }
   x->keep_prev = true;
@@ -2259,12 +2255,8 @@ int gnn_predict_launch(fpsi_gnn* m, fpsi_ctx* x, double* dx0, bool jacobi_in_ite
   if (rc) return rc;
   // from now on the context keeps a copy of each applied update
   if (!x->d_xprev) {
-    if (cudaMalloc(&x->d_xprev, size_t(nc) * 5 * 8) != cudaSuccess) {
-      x->d_xprev = nullptr;
-      set_error("cudaMalloc failed for the previous-update copy");
-      cudaGetLastError();
-      return FPSI_E_NOMEM;
-    }
+    const int rc = fpsi::device_alloc(x, (void**)&x->d_xprev, size_t(nc) * 5 * 8);
+    if (rc) return rc;
     x->have_xprev = false;
   }
   x->keep_prev = true;

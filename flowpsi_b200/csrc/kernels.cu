@@ -2334,12 +2334,17 @@ int launch_grad_records(fpsi_ctx* x) {
   return FPSI_OK;
 }
 
+static int alloc_material(fpsi_ctx* x) {
+  return x->d_muk ? FPSI_OK : device_alloc(x, (void**)&x->d_muk, size_t(x->H.nc) * 2 * sizeof(double));
+}
+
 int ensure_material(fpsi_ctx* x) {
   const double m[6] = {x->P.mu_a1, x->P.mu_a2, x->P.mu_a3, x->P.k_a1, x->P.k_a2, x->P.k_a3};
   bool same = x->muk_valid;
   for (int i = 0; i < 6; ++i) same = same && x->muk_with[i] == m[i];
   if (same) return FPSI_OK;
-  if (!x->d_muk) FPSI_CUDA_TRY(cudaMalloc(&x->d_muk, size_t(x->H.nc) * 2 * sizeof(double)));
+  int rc;
+  if ((rc = alloc_material(x))) return rc;
   dev::k_material<<<blocks_for(x->H.nc, 256), 256, 0, x->stream>>>(x->H.nc, x->d_q, visc(x));
   FPSI_CUDA_TRY(cudaGetLastError());
   note_material(x);
@@ -2355,6 +2360,7 @@ int launch_residual(fpsi_ctx* x, const NormOut& norms) {
   const dev::Gas g = gas(x);
   cudaStream_t s = x->stream;
   const int T = 256;
+  int rc;
   if (x->H.nbf > 0) {
     prof_begin(x, "bc_state");
     if (x->any_pmean)
@@ -2365,10 +2371,10 @@ int launch_residual(fpsi_ctx* x, const NormOut& norms) {
   }
   const bool kec = x->P.flux == FPSI_FLUX_KEC || x->P.flux == FPSI_FLUX_SSF;
   if (kec) {
-    if (!x->d_adiss) {
-      FPSI_CUDA_TRY(cudaMalloc(&x->d_adiss, size_t(M.nc) * sizeof(double)));
-      FPSI_CUDA_TRY(cudaMalloc(&x->d_ageom, size_t(std::max<int64_t>(M.nfi, 1)) * sizeof(float)));
-    }
+    if (!x->d_adiss && (rc = device_alloc(x, (void**)&x->d_adiss, size_t(M.nc) * sizeof(double)))) return rc;
+    if (!x->d_ageom &&
+        (rc = device_alloc(x, (void**)&x->d_ageom, size_t(std::max<int64_t>(M.nfi, 1)) * sizeof(float))))
+      return rc;
     if (x->ageom_coeff != x->P.lds_nonsym_coeff || x->ageom_factor != x->P.lds_nonsym_factor) {
       if (M.nfi > 0)
         dev::k_alpha_geom<<<blocks_for(M.nfi, T), T, 0, s>>>(M, lds(x), x->d_ageom);
@@ -2378,7 +2384,7 @@ int launch_residual(fpsi_ctx* x, const NormOut& norms) {
   }
   // the laws kept are an older state's from here on, until a kernel fills them
   x->muk_valid = false;
-  if (x->P.viscous && !x->d_muk) FPSI_CUDA_TRY(cudaMalloc(&x->d_muk, size_t(M.nc) * 2 * sizeof(double)));
+  if (x->P.viscous && (rc = alloc_material(x))) return rc;
   prof_begin(x, "grad_limiter");
   // the gradient records are written every residual only where the viscous
   // terms, the SA model and the KEC flux read them

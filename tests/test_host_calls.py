@@ -331,3 +331,45 @@ for name, sa, f in [
                 assert any(d.what == "sync" and d.stream == c.stream for d in calls[i:]), (name, k, c)
 assert tried > 30, tried
 """)
+
+
+def test_the_reported_device_memory_is_what_is_held():
+    """fpsi_info's device_bytes: arrays made on first use and arrays given
+    back when options change included"""
+    run("""
+from flowpsi_b200 import _native as N
+from flowpsi_b200.learned import LearnedStart
+size = [0]  # what the context has asked for
+def look(c):
+    if c.what == "malloc":
+        size[0] += c.n
+    return 0
+def reported(g):
+    b = C.c_int64()
+    N.lib().fpsi_info(g._ctx, None, None, None, C.byref(b))
+    return b.value
+c = cases.boundary_layer_block(4, 6, 3, dy0=1e-3, growth=1.3, viscous=2, precision="ref", sa=True)
+on.append(look)
+g = FlowPsi(c.mesh, c.params)
+assert reported(g) == size[0]
+g.set_state(*c.initial_state(g.geometry()["cellcenter"]))
+g.residual(); g.assemble(); g.linear_solve(); g.sa_residual(); g.run(4)
+assert reported(g) == size[0]  # the cells' viscosities among it
+p = g.params
+p.flux, p.viscous, p.turbulence, p.solver = 3, 0, 0, 0
+g.set_params(p); g.residual(); g.assemble(); g.linear_solve()
+assert reported(g) == size[0]
+n0 = reported(g)
+g.keep_blocks(False); g.keep_blocks(True)
+assert reported(g) == n0       # given back and made again
+p.precision = 0
+g.set_params(p)
+assert n0 < reported(g) < 2 * n0
+p.precision = 1
+g.set_params(p)
+assert reported(g) == n0
+g.residual(); g.assemble()
+m = LearnedStart(seed=0)
+m.predict(g)
+assert reported(g) == n0 + 5 * 8 * g.ncells + 4 * (g.ncells + 1) + 4 * 2 * int((c.mesh.arrays().cr >= 0).sum())
+""")
