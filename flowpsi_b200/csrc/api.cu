@@ -338,6 +338,10 @@ int rows_up(fpsi_ctx* x, int w, const int32_t* map, const double* in, void* dst,
 
 extern "C" {
 
+namespace {
+void batch_trim();  // of the batched face calls, below
+}
+
 void fpsi_default_params(fpsi_params* p) {
   if (!p) return;
   std::memset(p, 0, sizeof(*p));
@@ -421,6 +425,7 @@ int fpsi_destroy(fpsi_ctx* x) {
   for (cudaEvent_t e : x->evpool) cudaEventDestroy(e);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete x;
+  batch_trim();
   return FPSI_OK;
 }
 
@@ -1448,7 +1453,7 @@ namespace {
 // Device scratch of the batched calls: a stream-ordered pool per device, which
 // keeps up to BATCH_KEEP bytes between calls and gives the rest back when the
 // device is next synchronised (a call's five cudaMalloc and cudaFree took 0.6
-// of its 0.75 ms at 2,000 faces).  The driver hands out and reuses the memory,
+// of its 0.75 ms at 2,000 faces).  fpsi_destroy gives back what is kept.  The driver hands out and reuses the memory,
 // so calls from several threads are safe.
 // A pool belongs to the device's context: after a cudaDeviceReset the context
 // has another id and the next call makes a new pool.
@@ -1500,6 +1505,22 @@ int batch_pool(cudaMemPool_t* pool) {
   }
   *pool = b.pool;
   return FPSI_OK;
+}
+
+// the current device's kept memory back to the driver (what a call in another
+// thread holds stays)
+void batch_trim() {
+  int dev = 0;
+  unsigned long long id = 0;
+  std::lock_guard<std::mutex> lock(batch_mutex);
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= BATCH_DEVICES || !batch_pools[dev].pool ||
+      !context_id(&id) || id != batch_pools[dev].context) {
+    cudaGetLastError();
+    return;
+  }
+  cudaStreamSynchronize(cudaStreamLegacy);  // the calls' frees
+  cudaMemPoolTrimTo(batch_pools[dev].pool, 0);
+  cudaGetLastError();
 }
 
 // the inputs of n faces on the device (qL, qR, normals, areas) and room for

@@ -491,7 +491,9 @@ int fpsi_residual_norms_noalloc(const double* d_src, const double* d_vol, int64_
 
 /* ---- face functions on batches (inviscidFlux.h entry points) --------------
  * States are packed per face as [pg, T, u, v, w] (n*5), normals n*3 (unit),
- * area n.  Host pointers; copies and one kernel launch inside. */
+ * area n.  Host pointers; copies and one kernel launch inside.
+ * The calls keep up to 128 MB of device memory per device for the next one;
+ * fpsi_destroy of any context on that device gives it back. */
 int fpsi_face_flux(int32_t kind, int64_t n, const double* qL, const double* qR,
                    const double* an, const double* area, double pambient,
                    double Rt, double gamma, double us_n, double eta, double* flux);
