@@ -200,7 +200,8 @@ int alloc_lsgs(fpsi_ctx* x) {
   if ((rc = dalloc(x, (char**)&x->d_lctl, 64))) return rc;
   if ((rc = dalloc(x, &x->d_lpart, (nt + 255) / 256 + 1))) return rc;
   // padding cells must read as zero in the relaxation and the residual, and
-  // couplings past a line's ends as zero in the line solves
+  // couplings past a line's ends as zero in the line solves (k_lsgs_scatter
+  // says what relies on it)
   FPSI_CUDA_TRY(cudaMemset(x->d_lD, 0, nt * 30 * td));
   FPSI_CUDA_TRY(cudaMemset(x->d_lL, 0, nt * 25 * tb));
   FPSI_CUDA_TRY(cudaMemset(x->d_lU, 0, nt * 25 * tb));

@@ -1817,7 +1817,10 @@ constexpr int SGS_THREADS = 128;
 // against 0.296 slot by slot) and for FP32 tets of any size (663,552 cells:
 // 1.050 against 1.053, 1.57 M 2.481 against 2.525); larger grids of the
 // other forms stream faster slot by slot (592,704 hexes MIXED 1.00 against
-// 1.09, 663,552 tets FP64 1.65 against 1.90).
+// 1.09, 663,552 tets FP64 1.65 against 1.90).  For REF tets past one wave (a
+// symmetric sweep by itself): 663,552 cells 94 us slot by slot against 102,
+// 1.57 M 225 against 230, 384,000 58 against 59; only just past it does the
+// other form win (131,712 cells, 1.02 waves: 34 against 31 us).
 template <class TB, class TX, bool CPT, int MS>
 constexpr int sgs_ahead() {
   return MS == 0 ? 0 : sizeof(TB) == 4 ? (CPT ? 4 : 2) : (CPT ? 1 : 0);

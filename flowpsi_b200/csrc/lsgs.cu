@@ -300,8 +300,15 @@ constexpr int DROW = 30 * 32;
 // (row p to p-1 in L, to p+1 in U), outer couplings and B.  The coupling of
 // row c to neighbour n through face f is fjm_f when c = cl(f), -fjp_f when
 // c = cr(f) (solverLinearSystem.loci:57-77).  One thread per line slot t,
-// so that the 32 lanes of a row store 32 consecutive words of every stream;
-// padding slots are left as they are (never read as data).
+// so that the 32 lanes of a row store 32 consecutive words of every stream.
+//
+// What is not written here has to stay as alloc_lsgs cleared it.  The line
+// solves walk a group's rows for all 32 lanes and have no test at a line's
+// ends: U of a line's last row, which they multiply with the zero that starts
+// the back substitution, must be zero (and so finite), L of a first row is
+// copied along; D, L and U of padding rows are computed on, with the results
+// dropped.  Nothing else may use these arrays.  The first coupling of a slot
+// without any (lF) is read ahead and dropped, whatever it holds.
 template <class TB, class TD>
 __global__ void k_lsgs_scatter(int64_t nt, const int32_t* __restrict__ c_of_t,
                                const int32_t* __restrict__ cf_off, const int32_t* __restrict__ cf,
@@ -418,8 +425,10 @@ __device__ __forceinline__ void lu5_nopiv_recip(T* A, T* r, uint32_t& key) {
 // (the pivots' reciprocals, which the solves need as well); the others are
 // quotient()s.  A row whose operands leave their range, or that comes out
 // not finite, is done again with divisions.  262,144 cells in rows of 64:
-// 134 -> 70 us MIXED; 24,576 cells in rows of 32: 114 -> 76 us REF, 109 -> 82 us
-// FP64 (whose next row's blocks do not fit beside this one's).
+// 134 -> 70 us MIXED; 24,576 cells in rows of 32: 114 -> 78 us REF, 109 -> 84 us
+// FP64 (whose next row's blocks do not fit beside this one's).  The FP64 forms
+// spend 2 to 15 us of 84 to 226 on telling the smallest subnormal dividends from
+// zero (line_quotient.cuh).
 template <class TB, class TD>
 __global__ void k_lsgs_prep(int64_t ngroups, LineView V, TD* __restrict__ lD,
                             const TB* lL, const TB* lU,
@@ -625,9 +634,10 @@ constexpr size_t thomas_smem_bytes(int nst, int64_t rows) {
 // rows whose operands leave its range is done again with divisions.  An LSGS
 // iteration of 131,072 cells (64 rows, four solves with their right-hand
 // sides, MIXED) went from 397 to 174 us: a row's step from 0.66 to 0.21 us,
-// against about 0.1 us of its dependent FMAs.  Every wait is bounded; one that gives
-// up sets bit 4 of err and the abort flag, and the copies in flight land
-// before the CTA ends.
+// against about 0.1 us of its dependent FMAs (the iteration is 156 us with the
+// launches overlapped; 154 where each lane decided on its wait alone).  Every
+// wait is bounded and its outcome the warp's; one that gives up sets bit 4 of
+// err and the abort flag, and the copies in flight land before the CTA ends.
 template <class TB, class TD, class TX, bool YS>
 __global__ void __launch_bounds__(THOMAS_THREADS)
 k_lsgs_thomas(int nst, int64_t g0, LineView V, const TD* lD, const TB* lL,
