@@ -312,11 +312,13 @@ void unpermute_cells(const fpsi_ctx* x, const T* dev_order, int w, T* caller) {
   }
 }
 
-// the end of a call that may have queued copies of the caller's arrays: they
-// are not in flight any more when it returns, with an error neither
+// the end of a call that may have queued copies of the caller's arrays, or
+// steps that write the history: nothing of it is in flight any more when it
+// returns, with an error neither
 int finish(fpsi_ctx* x, int rc) {
   if (!rc) return sync(x);
   cudaStreamSynchronize(x->stream);
+  cudaGetLastError();  // rc says it
   return rc;
 }
 
@@ -1355,8 +1357,7 @@ int fpsi_run(fpsi_ctx* x, int32_t nsteps, fpsi_resid* norms) {
   int rc = ensure_hist(x, nsteps);
   if (rc) return rc;
   int32_t launched = 0;
-  rc = run_steps(x, nsteps, &launched);
-  if (!rc) rc = sync(x);
+  rc = finish(x, run_steps(x, nsteps, &launched));
   x->have_resid = x->have_asm = x->have_dq = false;
   if (rc) return rc;
   return finish_run(x, nsteps, launched, norms);
@@ -1372,8 +1373,7 @@ int fpsi_time_step(fpsi_ctx* x, fpsi_resid* norms) {
   int rc = ensure_hist(x, nit);
   if (rc) return rc;
   int32_t launched = 0;
-  rc = run_steps(x, nit, &launched);
-  if (!rc) rc = sync(x);
+  rc = finish(x, run_steps(x, nit, &launched));
   x->have_resid = x->have_asm = x->have_dq = false;
   if (rc) return rc;
   if ((rc = finish_run(x, nit, launched, norms))) return rc;
@@ -1394,7 +1394,7 @@ int fpsi_run_timed(fpsi_ctx* x, int32_t nsteps, fpsi_resid* norms, double* devic
   int32_t launched = 0;
   if (!rc) rc = run_steps(x, nsteps, &launched);
   if (!rc && cudaEventRecord(b, x->stream) != cudaSuccess) rc = FPSI_E_CUDA;
-  if (!rc) rc = sync(x);
+  rc = finish(x, rc);
   float ms = 0;
   if (!rc && cudaEventElapsedTime(&ms, a, b) != cudaSuccess) rc = FPSI_E_CUDA;
   if (a) cudaEventDestroy(a);
@@ -1414,9 +1414,8 @@ int fpsi_kernel_times(fpsi_ctx* x, int32_t nsteps, int32_t cap, char* names, dou
   x->evnext = 0;
   x->profiling = true;
   int32_t launched = 0;
-  rc = run_steps(x, nsteps, &launched);
+  rc = finish(x, run_steps(x, nsteps, &launched));
   x->profiling = false;
-  if (!rc) rc = sync(x);
   x->have_resid = x->have_asm = x->have_dq = false;
   if (rc) return rc;
   if ((rc = finish_run(x, nsteps, launched, nullptr))) return rc;

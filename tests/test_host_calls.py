@@ -373,3 +373,36 @@ m = LearnedStart(seed=0)
 m.predict(g)
 assert reported(g) == n0 + 5 * 8 * g.ncells + 4 * (g.ncells + 1) + 4 * 2 * int((c.mesh.arrays().cr >= 0).sum())
 """)
+
+
+def test_a_failed_run_waits_for_the_steps_in_flight():
+    """the steps write their norms to pinned memory that the next, longer run
+    gives back"""
+    run("""
+c = cases.farfield_cube(4, precision="ref")
+c.params.time_accurate, c.params.newton_iters = 1, 4
+g = FlowPsi(c.mesh, c.params)
+st = c.initial_state(g.geometry()["cellcenter"])
+s = None
+for f in (lambda: g.run(6), lambda: g.time_step(), lambda: g.run_timed(6), lambda: g.kernel_times(2)):
+    for what, k in (("launch", 5), ("graph", 2)):
+        g.set_state(*st)
+        del calls[:]
+        n = [0]
+        def refuse(c):
+            n[0] += c.what == what
+            return 700 if c.what == what and n[0] == k else 0
+        on.append(refuse)
+        try:
+            f()
+            failed = False
+        except FpsiError:
+            failed = True
+        on.remove(refuse)
+        if n[0] < k:
+            continue  # no graphs in this call
+        assert failed, what
+        last = max(i for i, c in enumerate(calls) if c.what in ("launch", "graph"))
+        stream = calls[last].stream
+        assert any(c.what == "sync" and c.stream == stream for c in calls[last:]), (what, [c[:2] for c in calls[last:]])
+""")
